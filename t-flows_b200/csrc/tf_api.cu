@@ -187,6 +187,12 @@ int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes) {
   return TF_OK;
 }
 
+void tf_dev_free(tf_ctx_s* ctx, void* p) {
+  if (!p) return;
+  if (ctx->async_alloc) cudaFreeAsync(p, ctx->stream);
+  else cudaFree(p);
+}
+
 void tf_matrix_free(tf_matrix_s* m) {
   if (!m) return;
   cudaSetDevice(m->ctx->device);
@@ -199,14 +205,11 @@ void tf_matrix_free(tf_matrix_s* m) {
   void* ptrs[] = {m->d_row, m->d_col, m->d_dia, m->d_tiles, m->d_val, m->d_x, m->d_b,
                   m->d_r, m->d_p, m->d_q, m->d_z, m->d_adiag, m->d_part,
                   m->d_hist, m->d_state, m->d_params, m->d_levf_rows, m->d_levb_rows,
-                  m->d_icc_d, m->d_icc_dinv, m->d_icc_levf_ptr, m->d_icc_levb_ptr,
+                  m->d_icc_d, m->d_icc_dinv,
                   m->d_pat, m->d_pat_tab, m->d_perm, m->d_src,
                   m->d_face_cell, m->d_face_pos, m->d_cf_ptr, m->d_cf};
-  for (void* p : ptrs)
-    if (p) {
-      if (m->async_alloc) cudaFreeAsync(p, m->ctx->stream);
-      else cudaFree(p);
-    }
+  for (void* p : ptrs) tf_dev_free(m->ctx, p);
+  tf_icc_free(m);
   if (!m->host_lent) {
     if (m->h_state) cudaFreeHost(m->h_state);
     if (m->h_params) cudaFreeHost(m->h_params);
@@ -519,7 +522,8 @@ int matrix_create_impl(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const
       }
     }
     if (st == TF_OK) st = tf_choose_tiles(m, fit_mask);
-  }  if (st == TF_OK && n_cells > 0 && diag_first && want_icc)
+  }
+  if (st == TF_OK && n_cells > 0 && diag_first && want_icc)
     st = tf_icc_build(m, row0.data(), col0.data());
   if (st == TF_OK && allow_renumber) st = attach_renumbered(m, row0, col0, dia0);
   if (st != TF_OK) {

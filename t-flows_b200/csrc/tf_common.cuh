@@ -57,8 +57,15 @@ struct SolveState {
   int x_pend;         // x still lacks the last alpha * p (deferred update)
   int pad;
   unsigned counter[8];  // last-block-done counters, one per kernel kind
-  unsigned bar_count;   // grid barrier of the persistent ICC sweeps: arrivals
-  unsigned bar_gen;     // ... and generation
+};
+
+// Where a new residual is also stored for the one-CTA ICC sweeps: in the
+// records of both directions (tf_icc_plan.h; null pointers: nowhere).
+struct IccResid {
+  const int* idx_f;
+  const int* idx_b;
+  double* rec_f;
+  double* rec_b;
 };
 
 enum CounterSlot { kCntDiag = 0, kCntScale, kCntResid, kCntSpmv, kCntUpdate,
@@ -345,6 +352,29 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, unsigned parit
   while (!mbar_try_wait(bar, parity))
     if (*abort_flag || globaltimer_ns() > deadline) return false;
   return globaltimer_ns() <= deadline;
+}
+// A deadline that costs a clock register to look at: the global timer (about
+// a microsecond to read) is read at the first look and then only when
+// kLookCycles have passed since, so a limit is kept to within that.
+struct Deadline {
+  unsigned long long ns;   // globaltimer
+  long long look;          // SM clock at which to read it again
+  static constexpr long long kLookCycles = 16384;
+  __device__ __forceinline__ explicit Deadline(unsigned long long limit_ns)
+      : ns(deadline_after(limit_ns)), look(0) {}
+  __device__ __forceinline__ bool passed() {
+    const long long c = clock64();
+    if (c < look) return false;
+    look = c + kLookCycles;
+    return globaltimer_ns() > ns;
+  }
+};
+// mbar_wait_or_abort on such a deadline.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity,
+                                          volatile int* abort_flag, Deadline& deadline) {
+  while (!mbar_try_wait(bar, parity))
+    if (*abort_flag || deadline.passed()) return false;
+  return !deadline.passed();
 }
 // Wait for the bulk copies armed on `bar` before the CTA exits: always the
 // default limit (never the caller's), so a short caller limit cannot end a

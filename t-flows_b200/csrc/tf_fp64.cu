@@ -42,7 +42,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "tf_icc.cuh"
+#include "tf_icc_plan.h"
 #include "tf_internal.h"
 #include "tf_tile.cuh"
 #include "tf_tile2.cuh"
@@ -64,9 +64,18 @@ struct VecArgs {
   double* part;
   SolveState* st;
   const SolveParams* prm;
+  IccResid icc;       // kPrecIcc
   cudaGraphConditionalHandle cond;
   int use_cond;
 };
+
+template <int PREC>
+__device__ __forceinline__ void icc_residual(const IccResid& c, int i, double r) {
+  if (PREC == kPrecIcc && c.idx_f) {
+    c.rec_f[c.idx_f[i]] = r;
+    c.rec_b[c.idx_b[i] + 2] = r;
+  }
+}
 
 __device__ __forceinline__ void set_cond(const VecArgs& a, int v) {
   if (a.use_cond) cudaGraphSetConditional(a.cond, (unsigned)v);
@@ -105,7 +114,6 @@ __global__ void __launch_bounds__(256) k_diag(VecArgs a) {
     st->iter = 0;
     st->niter = 0;
     st->status = 0;
-    st->bar_count = 0u;   // a timed-out ICC sweep may have left arrivals behind
     st->res = 0.0;
     st->rho = 0.0;
     st->rho_old = 0.0;
@@ -236,6 +244,7 @@ struct OpResidual {
   const double* __restrict__ b;
   double* __restrict__ r;
   const double* __restrict__ adiag;
+  IccResid icc;
   double s, rho;
   template <class COL>
   __device__ __forceinline__ void body(int i, const double* v, COL col, int len) {
@@ -254,6 +263,7 @@ struct OpResidual {
         if (k0 + u < len) acc = __dsub_rn(acc, __dmul_rn(vv[u], xv[u]));
     }
     r[i] = acc;
+    icc_residual<PREC>(icc, i, acc);
     const double ai = adiag[i];
     s = __dadd_rn(s, nrms_term(acc, ai));
     if (PREC == kPrecJacobi) {
@@ -280,6 +290,7 @@ struct OpResidual {
   }
   __device__ __forceinline__ void row_done(int i, double acc) {
     r[i] = acc;
+    icc_residual<PREC>(icc, i, acc);
     const double ai = adiag[i];
     s = __dadd_rn(s, nrms_term(acc, ai));
     if (PREC == kPrecJacobi) {
@@ -402,7 +413,7 @@ __global__ void __launch_bounds__(cfg_threads<CFG, PAT>(), cfg_min_blocks<CFG, P
   __shared__ double scratch[32];
   SolveState* st = a.v.st;
   if (st && st->done) return;
-  OpResidual<PREC> op{a.v.x, a.v.b, a.v.r, a.v.adiag, 0.0, 0.0};
+  OpResidual<PREC> op{a.v.x, a.v.b, a.v.r, a.v.adiag, a.v.icc, 0.0, 0.0};
   if (!run_rows<CFG, PAT>(a, op) && threadIdx.x == 0) flag_timeout(st);
   double v[2] = {block_red<kSum>(op.s, scratch), block_red<kSum>(op.rho, scratch)};
   const int ops[2] = {kSum, kSum};
@@ -598,13 +609,17 @@ __global__ void __launch_bounds__(256, 3) k_update(VecArgs a) {
         o.x = row(rv[u].x, qv[u].x, av[u].x);
         o.y = row(rv[u].y, qv[u].y, av[u].y);
         r2[jj] = o;
+        icc_residual<PREC>(a.icc, 2 * jj, o.x);
+        icc_residual<PREC>(a.icc, 2 * jj + 1, o.y);
       }
     }
   }
   if ((a.ni & 1) && tid == 0) {   // the odd last row
     const int i = a.ni - 1;
     if (!XDEF) a.x[i] = xrow(a.x[i], a.p[i]);
-    a.r[i] = row(a.r[i], a.q[i], a.adiag[i]);
+    const double ri = row(a.r[i], a.q[i], a.adiag[i]);
+    a.r[i] = ri;
+    icc_residual<PREC>(a.icc, i, ri);
   }
   double v[4] = {s, rho, mn, mx};
   const int ops[4] = {kSum, kSum, kMin, kMax};
@@ -700,6 +715,7 @@ VecArgs make_vec_args(tf_matrix_s* m) {
   a.part = m->d_part;
   a.st = m->d_state;
   a.prm = m->d_params;
+  a.icc = tf_icc_resid(m);
   a.cond = 0;
   a.use_cond = 0;
   return a;
@@ -742,88 +758,6 @@ struct NodeBuilder {
     }
     return node;
   }
-  // A kernel node launched cooperatively (all its CTAs resident at once).
-  cudaGraphNode_t add_coop(const void* fn, dim3 grid, dim3 block, void** args,
-                           cudaGraphNode_t dep) {
-    cudaGraphNode_t node = add(fn, grid, block, 0, args, dep);
-    if (status != TF_OK) return nullptr;
-    cudaKernelNodeAttrValue v{};
-    v.cooperative = 1;
-    cudaError_t e = cudaGraphKernelNodeSetAttribute(node, cudaKernelNodeAttributeCooperative, &v);
-    if (e != cudaSuccess) {
-      tf_set_last_cuda_error(e, "cudaGraphKernelNodeSetAttribute(cooperative)", __FILE__,
-                             __LINE__);
-      status = TF_ERR_CUDA;
-    }
-    return node;
-  }
-};
-
-// Arguments of the persistent ICC sweeps.
-struct IccSweeps {
-  IccSweepArgs form, fwd, bwd;
-};
-IccArgs icc_args(tf_matrix_s* m);
-IccSweeps icc_sweep_args(tf_matrix_s* m) {
-  IccSweeps w{};
-  IccArgs a = icc_args(m);
-  a.rows = m->d_levf_rows;
-  w.fwd = IccSweepArgs{a, m->d_icc_levf_ptr, (int)m->h_levf_ptr.size() - 1, m->d_state,
-                       m->d_params};
-  w.form = w.fwd;
-  w.form.a.st = nullptr;
-  a.rows = m->d_levb_rows;
-  w.bwd = IccSweepArgs{a, m->d_icc_levb_ptr, (int)m->h_levb_ptr.size() - 1, m->d_state,
-                       m->d_params};
-  return w;
-}
-
-IccArgs icc_args(tf_matrix_s* m) {
-  IccArgs a{};
-  a.row = m->d_row;
-  a.col = m->d_col;
-  a.val = m->d_val;
-  a.ni = m->ni;
-  a.d = m->d_icc_d;
-  a.d_inv = m->d_icc_dinv;
-  a.r = m->d_r;
-  a.y = m->d_q;   // q is free between k_update and the next SpMV
-  a.z = m->d_z;
-  a.st = m->d_state;
-  return a;
-}
-
-// Per-level kernel arguments, kept alive while a graph is built.
-struct IccLevelArgs {
-  std::vector<IccArgs> form, fwd, bwd;
-};
-
-IccLevelArgs icc_level_args(tf_matrix_s* m) {
-  IccLevelArgs L;
-  const IccArgs base = icc_args(m);
-  for (size_t l = 0; l + 1 < m->h_levf_ptr.size(); ++l) {
-    IccArgs a = base;
-    a.rows = m->d_levf_rows + m->h_levf_ptr[l];
-    a.count = m->h_levf_ptr[l + 1] - m->h_levf_ptr[l];
-    L.fwd.push_back(a);
-    a.st = nullptr;
-    L.form.push_back(a);
-  }
-  for (size_t l = 0; l + 1 < m->h_levb_ptr.size(); ++l) {
-    IccArgs a = base;
-    a.rows = m->d_levb_rows + m->h_levb_ptr[l];
-    a.count = m->h_levb_ptr[l + 1] - m->h_levb_ptr[l];
-    L.bwd.push_back(a);
-  }
-  return L;
-}
-
-struct RhoArgs {
-  int ni;
-  const double* z;
-  const double* r;
-  double* part;
-  SolveState* st;
 };
 
 // The iteration's vector kernels for this solve: xdef defers x += alfa p
@@ -867,51 +801,25 @@ int build_graph_t(tf_matrix_s* m, int xdef, cudaGraphExec_t* out) {
   NodeBuilder nb{g};
   void* vargs[] = {&va};
   void* sargs[] = {&sa};
-  IccLevelArgs lv;
-  RhoArgs ra{m->ni, m->d_z, m->d_r, m->d_part, m->d_state};
-  void* rargs[] = {&ra.ni, &ra.z, &ra.r, &ra.part, &ra.st};
-  std::vector<void*> form_args, fwd_args, bwd_args;
-  IccSweeps sw{};
-  void* sw_form[] = {&sw.form};
-  void* sw_fwd[] = {&sw.fwd};
-  void* sw_bwd[] = {&sw.bwd};
-  const bool sweeps = PREC == kPrecIcc && m->icc_sweep_grid > 0;
-  const dim3 swg(std::max(1, m->icc_sweep_grid));
+  tf_icc_plan icc;
   if (PREC == kPrecIcc) {
-    lv = icc_level_args(m);
-    sw = icc_sweep_args(m);
-    for (auto& a : lv.form) form_args.push_back(&a);
-    for (auto& a : lv.fwd) fwd_args.push_back(&a);
-    for (auto& a : lv.bwd) bwd_args.push_back(&a);
-  }
-  auto lgrid = [](int count) { return dim3(std::max(1, (count + 255) / 256)); };
-  // z = M^-1 r by the two triangular sweeps (persistent kernels, or one
-  // kernel per level), then rho = z.r
-  auto add_icc_apply = [&](NodeBuilder& b, cudaGraphNode_t dep) {
-    if (sweeps) {
-      dep = b.add_coop((const void*)k_icc_sweep<kSweepFwd>, swg, dim3(256), sw_fwd, dep);
-      dep = b.add_coop((const void*)k_icc_sweep<kSweepBwd>, swg, dim3(256), sw_bwd, dep);
-    } else {
-      for (size_t l = 0; l < lv.fwd.size(); ++l)
-        dep = b.add((const void*)k_icc_fwd_level, lgrid(lv.fwd[l].count), dim3(256), 0,
-                    &fwd_args[l], dep);
-      for (size_t l = 0; l < lv.bwd.size(); ++l)
-        dep = b.add((const void*)k_icc_bwd_level, lgrid(lv.bwd[l].count), dim3(256), 0,
-                    &bwd_args[l], dep);
+    st = tf_icc_make_plan(m, &icc);
+    if (st != TF_OK) {
+      cudaGraphDestroy(g);
+      return st;
     }
-    return b.add((const void*)k_icc_rho, vg, vb, 0, rargs, dep);
+  }
+  auto add_icc = [](NodeBuilder& b, std::vector<tf_icc_launch>& launches, cudaGraphNode_t dep) {
+    for (auto& l : launches)
+      dep = b.add(l.fn, dim3(l.grid), dim3(l.threads), l.smem, l.args.data(), dep);
+    return dep;
   };
   cudaGraphNode_t n1 = nb.add((const void*)k_diag, vg, vb, 0, vargs, nullptr);
   cudaGraphNode_t n2 = nb.add((const void*)k_scale, vg, vb, 0, vargs, n1);
-  if (PREC == kPrecIcc && sweeps)   // Prec_Form (Cg.f90:89) on the scaled matrix
-    n2 = nb.add_coop((const void*)k_icc_sweep<kSweepForm>, swg, dim3(256), sw_form, n2);
-  else if (PREC == kPrecIcc)
-    for (size_t l = 0; l < lv.form.size(); ++l)
-      n2 = nb.add((const void*)k_icc_form_level, lgrid(lv.form[l].count), dim3(256), 0,
-                  &form_args[l], n2);
+  if (PREC == kPrecIcc) n2 = add_icc(nb, icc.form, n2);   // Prec_Form (Cg.f90:89), scaled
   cudaGraphNode_t n3 = nb.add((const void*)k_residual<CFG, PREC, PAT>, sg, sb, ssm, sargs, n2);
   cudaGraphNode_t last = n3;
-  if (PREC == kPrecIcc) last = add_icc_apply(nb, last);
+  if (PREC == kPrecIcc) last = add_icc(nb, icc.apply, last);
   cudaGraphNode_t cnode = nullptr;
   if (nb.status == TF_OK) {
     cudaGraphNodeParams cp{};
@@ -929,7 +837,7 @@ int build_graph_t(tf_matrix_s* m, int xdef, cudaGraphExec_t* out) {
       cudaGraphNode_t b1 = body.add(fns.pupdate, vg, vb, 0, vargs, nullptr);
       cudaGraphNode_t b2 = body.add((const void*)k_spmv_alpha<CFG, PAT>, sg, sb, ssm, sargs, b1);
       cudaGraphNode_t b3 = body.add(fns.update, vg, vb, 0, vargs, b2);
-      if (PREC == kPrecIcc) add_icc_apply(body, b3);
+      if (PREC == kPrecIcc) add_icc(body, icc.apply, b3);
       if (body.status != TF_OK) nb.status = body.status;
     }
   }
@@ -979,29 +887,6 @@ int prepare_cfg(tf_matrix_s* m) {
 }
 
 }  // namespace
-
-int tf_icc_prepare_sweeps(tf_matrix_s* m) {
-  m->icc_sweep_grid = 0;
-  if (!getenv("TF_ICC_PERSISTENT")) return TF_OK;
-  int coop = 0;
-  TF_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->ctx->device));
-  if (!coop) return TF_OK;
-  int per_sm = 1 << 30;
-  for (const void* fn : {(const void*)k_icc_sweep<kSweepForm>, (const void*)k_icc_sweep<kSweepFwd>,
-                         (const void*)k_icc_sweep<kSweepBwd>}) {
-    int b = 0;
-    TF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 256, 0));
-    per_sm = std::min(per_sm, b);
-  }
-  if (per_sm < 1) return TF_OK;
-  // One CTA of 256 threads per SM: a level of a 200^3 hex grid has at most
-  // ~30,000 rows (about one per thread), and every CTA joins every barrier.
-  int widest = 1;
-  for (const auto* ptr : {&m->h_levf_ptr, &m->h_levb_ptr})
-    for (size_t l = 0; l + 1 < ptr->size(); ++l) widest = std::max(widest, (*ptr)[l + 1] - (*ptr)[l]);
-  m->icc_sweep_grid = std::max(1, std::min(m->ctx->sm_count, (widest + 255) / 256));
-  return TF_OK;
-}
 
 // ---------------------------------------------------------------------------
 // SpMV layout choice: the autotuner
@@ -1149,36 +1034,21 @@ int run_host_loop_t(tf_matrix_s* m, int xdef) {
   const size_t ssm = cfg_smem<CFG, PAT>();
   const IterFns fns = iter_fns<PREC>(xdef, m->vec_dir);
   void* vargs[] = {&va};
-  IccLevelArgs lv;
-  IccSweeps sw{};
-  const bool sweeps = PREC == kPrecIcc && m->icc_sweep_grid > 0;
+  tf_icc_plan icc;
   if (PREC == kPrecIcc) {
-    lv = icc_level_args(m);
-    sw = icc_sweep_args(m);
+    st = tf_icc_make_plan(m, &icc);
+    if (st != TF_OK) return st;
   }
-  auto lgrid = [](int count) { return std::max(1, (count + 255) / 256); };
-  auto coop = [&](const void* fn, IccSweepArgs* a) {
-    void* args[] = {a};
-    return cudaLaunchCooperativeKernel(fn, dim3(m->icc_sweep_grid), dim3(256), args, 0, s);
-  };
-  auto icc_apply = [&]() {
-    if (sweeps) {
-      coop((const void*)k_icc_sweep<kSweepFwd>, &sw.fwd);
-      coop((const void*)k_icc_sweep<kSweepBwd>, &sw.bwd);
-    } else {
-      for (auto& a : lv.fwd) k_icc_fwd_level<<<lgrid(a.count), 256, 0, s>>>(a);
-      for (auto& a : lv.bwd) k_icc_bwd_level<<<lgrid(a.count), 256, 0, s>>>(a);
-    }
-    k_icc_rho<<<vg, 256, 0, s>>>(m->ni, m->d_z, m->d_r, m->d_part, m->d_state);
+  auto icc_run = [&](std::vector<tf_icc_launch>& launches) -> int {
+    for (auto& l : launches)
+      TF_CUDA_TRY(cudaLaunchKernel(l.fn, dim3(l.grid), dim3(l.threads), l.args.data(), l.smem, s));
+    return TF_OK;
   };
   k_diag<<<vg, 256, 0, s>>>(va);
   k_scale<<<vg, 256, 0, s>>>(va);
-  if (PREC == kPrecIcc && sweeps)
-    TF_CUDA_TRY(coop((const void*)k_icc_sweep<kSweepForm>, &sw.form));
-  else if (PREC == kPrecIcc)
-    for (auto& a : lv.form) k_icc_form_level<<<lgrid(a.count), 256, 0, s>>>(a);
+  if (PREC == kPrecIcc && (st = icc_run(icc.form)) != TF_OK) return st;
   k_residual<CFG, PREC, PAT><<<sg, cfg_threads<CFG, PAT>(), ssm, s>>>(sa);
-  if (PREC == kPrecIcc) icc_apply();
+  if (PREC == kPrecIcc && (st = icc_run(icc.apply)) != TF_OK) return st;
   TF_CUDA_TRY(cudaGetLastError());
   constexpr int kChunk = 16;
   for (;;) {
@@ -1190,7 +1060,7 @@ int run_host_loop_t(tf_matrix_s* m, int xdef) {
       TF_CUDA_TRY(cudaLaunchKernel(fns.pupdate, dim3(vg), dim3(256), vargs, 0, s));
       k_spmv_alpha<CFG, PAT><<<sg, cfg_threads<CFG, PAT>(), ssm, s>>>(sa);
       TF_CUDA_TRY(cudaLaunchKernel(fns.update, dim3(vg), dim3(256), vargs, 0, s));
-      if (PREC == kPrecIcc) icc_apply();
+      if (PREC == kPrecIcc && (st = icc_run(icc.apply)) != TF_OK) return st;
     }
     TF_CUDA_TRY(cudaGetLastError());
   }
@@ -1212,6 +1082,10 @@ int tf_fp64_run(tf_matrix_s* m, int prec) {
   // x += alfa p can wait for the next k_pupdate when the NRMS does not
   // need the range of x (norm present); ICC keeps it in k_update.
   const int xdef = (prec != kPrecIcc && m->h_params->has_norm) ? 1 : 0;
+  if (prec == kPrecIcc) {
+    const int st = tf_icc_prepare(m);
+    if (st != TF_OK) return st;
+  }
   static const bool no_graph = getenv("TF_NO_GRAPH") != nullptr;
   if (no_graph) {
     if (prec == kPrecJacobi) return run_host_loop_p<kPrecJacobi>(m, xdef);

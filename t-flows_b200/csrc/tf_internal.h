@@ -86,6 +86,16 @@ struct tf_slice_s {
 };
 constexpr int kMaxRhs = 4;
 
+// One direction of the ICC sweeps on the device (tf::IccDir).
+struct tf_icc_dir_s {
+  int4* slice = nullptr;
+  int2* chunk = nullptr;
+  int* src = nullptr;
+  int* idx = nullptr;
+  unsigned char* rec = nullptr;
+  int nlev = 0, nslices = 0, far_any = 0;
+};
+
 // Device mirror of one Matrix_Type plus the Krylov workspace of its solves.
 struct tf_matrix_s {
   tf_ctx_s* ctx = nullptr;
@@ -135,10 +145,11 @@ struct tf_matrix_s {
   std::vector<int> h_levf_ptr, h_levb_ptr;
   double* d_icc_d = nullptr;     // Prec_Form's d
   double* d_icc_dinv = nullptr;  // Prec_Form's d_inv
-  // Persistent sweeps (k_icc_sweep): the level pointers on the device.
-  int* d_icc_levf_ptr = nullptr;
-  int* d_icc_levb_ptr = nullptr;
-  int icc_sweep_grid = 0;        // 0: per-level kernels
+  // The one-CTA sweeps' packed slices (tf_icc_prepare), made before the
+  // first ICC solve of a matrix with narrow levels.
+  tf_icc_dir_s icc_dir[2];       // forward, backward
+  int icc_packed = 0;
+  int icc_width = 0, icc_batch = 0, icc_warps = 0, icc_stages = 0, icc_ring = 0;
   // cached graphs, one per (preconditioner, x update deferred or not)
   cudaGraphExec_t graph[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   // The same graphs bound to a caller's device val/x/b (tf_solve_device in
@@ -195,12 +206,9 @@ int tf_fp64_residual(tf_matrix_s* m, const double* val, const double* b,
 int tf_fp64_nrms(tf_matrix_s* m, const double* val, const double* r,
                  const double* x, int has_norm, double norm, double* out);
 int tf_icc_build(tf_matrix_s* m, const int* h_row0, const int* h_col0);
-// Grid of the persistent ICC sweeps (tf_fp64.cu), which run only when
-// TF_ICC_PERSISTENT is set at registration (and the device launches
-// cooperatively): one kernel per level measured faster (a 120^3 hex: 4.8
-// against 5.3 ms per iteration).  icc_sweep_grid = 0 selects the per-level
-// kernels.
-int tf_icc_prepare_sweeps(tf_matrix_s* m);
+int tf_icc_prepare(tf_matrix_s* m);   // before a solve with ICC
+void tf_icc_free(tf_matrix_s* m);
+tf::IccResid tf_icc_resid(const tf_matrix_s* m);
 // Registration behind tf_matrix_register; want_icc = 0 skips the ICC level
 // schedule.  Device bytes the matrix will hold, for budgeting.
 int tf_matrix_create(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const int* row,
@@ -211,6 +219,7 @@ size_t tf_matrix_bytes(int n_cells, int64_t nnz);
 int tf_solve_resident(tf_matrix_s* m, int prec, int miter, double tol, const double* norm,
                       int* niter, double* fin_res);
 int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes);
+void tf_dev_free(tf_ctx_s* ctx, void* p);   // null is fine
 // Renumbering (tf_renumber.cu)
 double tf_gather_lines_per_warp(const int* row, const int* col, int n, int base);
 // Row patterns of the first ni rows of a 0-based CSR: pat[i] (ni + 32

@@ -273,9 +273,11 @@ class Matrix:
 
     def icc_launches_per_iteration(self):
         """Kernel launches of one ICC-preconditioned Cg iteration: the three
-        iteration kernels, one per sweep level, and the rho reduction."""
+        iteration kernels and the sweeps -- one kernel when the levels have at
+        most 2,000 rows on average, else one per level and the rho
+        reduction."""
         f, b = self.icc_levels()
-        return 3 + f + b + 1
+        return 4 if 2 * self.n_own <= 2000 * (f + b) else 3 + f + b + 1
 
     @property
     def renumbered(self):

@@ -614,3 +614,43 @@ def test_icc_needs_diagonal_first(gpu_ctx):
         assert native.solve(gpu_ctx, m, "cg", "jacobi", v, x, b, 10, 1e-8)[0] > 0
     finally:
         m.close()
+
+
+def _band_system(n, offsets, seed):
+    """Symmetric, diagonally dominant, diagonal first: row i is coupled to
+    i - o and i + o for every offset o."""
+    rng = np.random.default_rng(seed)
+    w = {o: rng.uniform(0.2, 1.0, n) for o in offsets}   # entry (i, i + o)
+    row, col, val = [1], [], []
+    for i in range(n):
+        ent = [(i + s * o, -w[o][i if s > 0 else i - o]) for o in offsets for s in (-1, 1)
+               if 0 <= i + s * o < n]
+        ent.sort()
+        col += [i + 1] + [j + 1 for j, _ in ent]
+        val += [0.3 - sum(v for _, v in ent)] + [v for _, v in ent]
+        row.append(len(col) + 1)
+    row = np.array(row, np.int32)
+    return row, np.array(col, np.int32), row[:-1].copy(), np.array(val), rng.uniform(-1, 1, n)
+
+
+@pytest.mark.parametrize("case", ["one-row", "slices", "hex-4-warps", "long-rows", "far",
+                                  "wide-levels"])
+def test_icc_sweeps_at_their_edges(gpu_ctx, case):
+    """The one-CTA sweeps where they can go wrong -- one row, levels of 31 to
+    33 rows, rows longer than the packed width (40 entries a side), results
+    older than the ring (9,000 positions back) -- and the kernel per level of
+    wide levels.  Row sums are the reference's, so the iterations are equal."""
+    if case in ("one-row", "slices", "hex-4-warps"):
+        from tflows_b200.grids import hex_grid
+        dims = {"one-row": (1, 1, 2), "slices": (33, 32, 3), "hex-4-warps": (17, 13, 11)}[case]
+        s = systems.pressure_system(hex_grid(*dims), 3, tol=1e-10, miter=500)
+        a = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b)
+    elif case == "long-rows":
+        a = _band_system(900, list(range(1, 41)), 5)
+    elif case == "far":
+        a = _band_system(12000, [4, 9000], 6)
+    else:   # two levels of 2,100 rows
+        a = _band_system(4200, [2100], 7)
+    n = len(a[4])
+    args = (*a, np.zeros(n), "cg", "icc", 300, 1e-10, 1.0)
+    check_parity(gpu_solve(gpu_ctx, *args), oracle_solve(*args), 1e-10, exact_iters=True)
