@@ -207,7 +207,7 @@ void tf_matrix_free(tf_matrix_s* m) {
                   m->d_hist, m->d_state, m->d_params, m->d_levf_rows, m->d_levb_rows,
                   m->d_icc_d, m->d_icc_dinv,
                   m->d_pat, m->d_pat_tab, m->d_perm, m->d_src,
-                  m->d_face_cell, m->d_face_pos, m->d_cf_ptr, m->d_cf};
+                  m->d_face_cell, m->d_face_pos, m->d_cf_ptr, m->d_cf, m->res.block};
   for (void* p : ptrs) tf_dev_free(m->ctx, p);
   tf_icc_free(m);
   if (!m->host_lent) {
@@ -526,6 +526,7 @@ int matrix_create_impl(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const
   if (st == TF_OK && n_cells > 0 && diag_first && want_icc)
     st = tf_icc_build(m, row0.data(), col0.data());
   if (st == TF_OK && allow_renumber) st = attach_renumbered(m, row0, col0, dia0);
+  if (st == TF_OK && n_cells > 0 && !m->ren) st = tf_resident_build(m, row0.data());
   if (st != TF_OK) {
     tf_matrix_free(m);
     return st;
@@ -635,11 +636,15 @@ int run_solve_core(tf_matrix_s* m, int prec, int miter, double tol,
     hp->hist = a->d_hist;
     hp->hist_cap = miter + 1;
   }
-  TF_CUDA_TRY(cudaMemcpyAsync(a->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));
   if (prec == tf::kPrecIcc && !m->icc_ready) return TF_ERR_LAYOUT;  // needs diagonal first
+  const bool resident = prec != tf::kPrecIcc && tf_resident(a);
+  if (!resident)
+    TF_CUDA_TRY(cudaMemcpyAsync(a->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));
   int st = TF_OK;
   if (a != m) st = tf_renumber_in(m);
-  if (st == TF_OK) st = tf_fp64_run(a, prec);
+  if (st == TF_OK)
+    st = resident ? tf_resident_run(a, prec, hp, a->d_x, a->d_b, a->d_state, 1)
+                  : tf_fp64_run(a, prec);
   if (st == TF_OK && a != m) st = tf_renumber_out(m);
   if (st != TF_OK) return st;
   TF_CUDA_TRY(cudaMemcpyAsync(m->h_state, a->d_state, sizeof(tf::SolveState),
@@ -651,7 +656,10 @@ int finish_solve(tf_matrix_s* m, int* niter, double* fin_res) {
   tf_ctx_s* c = m->ctx;
   TF_CUDA_TRY(cudaStreamSynchronize(c->stream));
   const tf::SolveState& s = *m->h_state;
-  if (s.status != 0) return s.status;
+  if (s.status != 0) {
+    const int st = tf_resident_reset(m->active ? m->active : m);
+    return st != TF_OK ? st : s.status;
+  }
   *niter = s.niter;
   *fin_res = s.res;
   c->last_count = 0;
@@ -805,10 +813,12 @@ const tf::SolveState* rhs_state(tf_matrix_s* m, int i) {
   return i == 0 ? m->d_state : m->slices[i - 1]->d_state;
 }
 
-// Runs the multi-RHS graph on the workspace (val, x_i, b_i already there)
-// and fetches the states; the caller copies results and synchronises.
+// Runs the multi-RHS graph on the workspace (val, x_i, b_i already there) --
+// or, on a resident matrix, its solves one after another on val and the given
+// x and b (null: the workspace's) -- and fetches the states; the caller copies
+// results and synchronises.
 int run_multi_core(tf_matrix_s* m, int prec, int nrhs, int miter, double tol,
-                   const double* norm) {
+                   const double* norm, double* x, double* b) {
   tf_ctx_s* c = m->ctx;
   tf::SolveParams* hp = m->h_params;
   hp->tol = tol;
@@ -818,8 +828,17 @@ int run_multi_core(tf_matrix_s* m, int prec, int nrhs, int miter, double tol,
   hp->hist = nullptr;
   hp->hist_cap = 0;
   hp->wait_ns = c->wait_ns;
-  TF_CUDA_TRY(cudaMemcpyAsync(m->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));
-  int st = tf_fp64_run_multi(m, prec, nrhs);
+  int st = TF_OK;
+  if (tf_resident(m)) {
+    for (int i = 0; i < nrhs && st == TF_OK; ++i)
+      st = tf_resident_run(m, prec, hp, x ? x + (size_t)i * m->nt : rhs_x(m, i),
+                           b ? b + (size_t)i * m->nt : rhs_b(m, i),
+                           const_cast<tf::SolveState*>(rhs_state(m, i)), i == nrhs - 1);
+  } else {
+    TF_CUDA_TRY(
+        cudaMemcpyAsync(m->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));
+    st = tf_fp64_run_multi(m, prec, nrhs);
+  }
   if (st != TF_OK) return st;
   if (!m->h_mstate) {
     cudaError_t e = cudaMallocHost((void**)&m->h_mstate, kMaxRhs * sizeof(tf::SolveState));
@@ -837,7 +856,10 @@ int run_multi_core(tf_matrix_s* m, int prec, int nrhs, int miter, double tol,
 int finish_multi(tf_matrix_s* m, int nrhs, int* niter, double* fin_res) {
   TF_CUDA_TRY(cudaStreamSynchronize(m->ctx->stream));
   for (int i = 0; i < nrhs; ++i)
-    if (m->h_mstate[i].status != 0) return m->h_mstate[i].status;
+    if (m->h_mstate[i].status != 0) {
+      const int st = tf_resident_reset(m);
+      return st != TF_OK ? st : m->h_mstate[i].status;
+    }
   for (int i = 0; i < nrhs; ++i) {
     niter[i] = m->h_mstate[i].niter;
     fin_res[i] = m->h_mstate[i].res;
@@ -879,7 +901,7 @@ extern "C" int tf_solve_multi(tf_ctx ctx, tf_matrix m, int solver, int prec, int
     TF_CUDA_TRY(cudaMemcpyAsync(rhs_b(m, i), b + (size_t)i * m->nt, nb,
                                 cudaMemcpyHostToDevice, s));
   }
-  st = run_multi_core(m, prec, nrhs, miter, tol, norm);
+  st = run_multi_core(m, prec, nrhs, miter, tol, norm, nullptr, nullptr);
   if (st != TF_OK) {
     cudaStreamSynchronize(s);
     return st;
@@ -909,17 +931,28 @@ extern "C" int tf_solve_multi_device(tf_ctx ctx, tf_matrix m, int solver, int pr
   if (!d_val || !d_x || !d_b) return TF_ERR_ARG;
   std::lock_guard<std::mutex> lk(m->mu);
   TF_CUDA_TRY(cudaSetDevice(ctx->device));
-  st = tf_slices_ensure(m, nrhs);
+  st = tf_slices_ensure(m, nrhs, tf_resident(m));
   if (st != TF_OK) return st;
   cudaStream_t s = ctx->stream;
   const size_t vb = (size_t)m->nnz * sizeof(double), nb = (size_t)m->nt * sizeof(double);
+  if (tf_resident(m)) {   // on the caller's arrays
+    double* own = m->d_val;
+    m->d_val = d_val;
+    st = run_multi_core(m, prec, nrhs, miter, tol, norm, d_x, d_b);
+    m->d_val = own;
+    if (st != TF_OK) {
+      cudaStreamSynchronize(s);
+      return st;
+    }
+    return finish_multi(m, nrhs, niter, fin_res);
+  }
   const cudaMemcpyKind dd = cudaMemcpyDeviceToDevice;
   TF_CUDA_TRY(cudaMemcpyAsync(m->d_val, d_val, vb, dd, s));
   for (int i = 0; i < nrhs; ++i) {
     TF_CUDA_TRY(cudaMemcpyAsync(rhs_x(m, i), d_x + (size_t)i * m->nt, nb, dd, s));
     TF_CUDA_TRY(cudaMemcpyAsync(rhs_b(m, i), d_b + (size_t)i * m->nt, nb, dd, s));
   }
-  st = run_multi_core(m, prec, nrhs, miter, tol, norm);
+  st = run_multi_core(m, prec, nrhs, miter, tol, norm, nullptr, nullptr);
   if (st != TF_OK) {
     cudaStreamSynchronize(s);
     return st;

@@ -357,11 +357,16 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, unsigned parit
 // a microsecond to read) is read at the first look and then only when
 // kLookCycles have passed since, so a limit is kept to within that.
 struct Deadline {
-  unsigned long long ns;   // globaltimer
-  long long look;          // SM clock at which to read it again
+  unsigned long long limit, ns;   // globaltimer
+  long long look;                 // SM clock at which to read it again
   static constexpr long long kLookCycles = 16384;
   __device__ __forceinline__ explicit Deadline(unsigned long long limit_ns)
-      : ns(deadline_after(limit_ns)), look(0) {}
+      : limit(limit_ns), ns(deadline_after(limit_ns)), look(0) {}
+  // The limit counts from now.
+  __device__ __forceinline__ void renew() {
+    ns = deadline_after(limit);
+    look = 0;
+  }
   __device__ __forceinline__ bool passed() {
     const long long c = clock64();
     if (c < look) return false;

@@ -1,5 +1,6 @@
 // tf_fp64.cu -- FP64 drop-in for Native_Mod's Cg and Bicg (Jacobi / none /
-// ICC preconditioning) on one B200.
+// ICC preconditioning) on one B200.  (Jacobi / none solves of matrices that
+// fit the chip run as one kernel instead: tf_resident.cu.)
 //
 // One solve is one CUDA graph:
 //
@@ -1453,17 +1454,18 @@ int build_multi_graph_p(tf_matrix_s* m, int nr, int xdef, cudaGraphExec_t* out) 
   });
 }
 
-int alloc_slice(tf_matrix_s* m, tf_slice_s** out) {
-  auto* s = new tf_slice_s();
-  const size_t nv = ((size_t)m->nt + 8) * sizeof(double);
+int alloc_slice(tf_matrix_s* m, tf_slice_s** out, bool state_only) {
+  if (!*out) *out = new tf_slice_s();
+  tf_slice_s* s = *out;
   int st = TF_OK;
+  if (!s->d_state) st = tf_dev_alloc_bytes(m->ctx, (void**)&s->d_state, sizeof(SolveState));
+  if (state_only) return st;
+  const size_t nv = ((size_t)m->nt + 8) * sizeof(double);
   for (double** p : {&s->d_x, &s->d_b, &s->d_r, &s->d_p, &s->d_q, &s->d_adiag})
-    if (st == TF_OK) st = tf_dev_alloc_bytes(m->ctx, (void**)p, nv);
-  if (st == TF_OK)
+    if (st == TF_OK && !*p) st = tf_dev_alloc_bytes(m->ctx, (void**)p, nv);
+  if (st == TF_OK && !s->d_part)
     st = tf_dev_alloc_bytes(m->ctx, (void**)&s->d_part,
                             ((size_t)8 * kMaxBlocks + 16) * sizeof(double));
-  if (st == TF_OK) st = tf_dev_alloc_bytes(m->ctx, (void**)&s->d_state, sizeof(SolveState));
-  *out = s;
   return st;
 }
 
@@ -1494,13 +1496,12 @@ void tf_slices_free(tf_matrix_s* m) {
   }
 }
 
-int tf_slices_ensure(tf_matrix_s* m, int nr) {
+int tf_slices_ensure(tf_matrix_s* m, int nr, bool states_only) {
   if (nr < 1 || nr > kMaxRhs) return TF_ERR_ARG;
-  for (int i = 0; i + 1 < nr; ++i)
-    if (!m->slices[i]) {
-      const int st = alloc_slice(m, &m->slices[i]);
-      if (st != TF_OK) return st;
-    }
+  for (int i = 0; i + 1 < nr; ++i) {
+    const int st = alloc_slice(m, &m->slices[i], states_only);
+    if (st != TF_OK) return st;
+  }
   return TF_OK;
 }
 

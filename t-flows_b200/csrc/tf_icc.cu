@@ -291,6 +291,10 @@ IccResid tf_icc_resid(const tf_matrix_s* m) {
   return r;
 }
 
+size_t tf_icc_bytes(int n, int64_t nnz) {
+  return (size_t)nnz * 18 + (size_t)n * 72 + ((size_t)1 << 16);
+}
+
 int tf_icc_prepare(tf_matrix_s* m) { return narrow_levels(m) ? pack(m) : TF_OK; }
 
 void tf_icc_free(tf_matrix_s* m) {

@@ -96,6 +96,22 @@ struct tf_icc_dir_s {
   int nlev = 0, nslices = 0, far_any = 0;
 };
 
+// The matrix's distribution over the CTAs of the resident solve
+// (tf_resident.cu); ctas = 0: it does not fit the chip.
+struct tf_resident_s {
+  int ctas = 0, shape = 0, threads = 0;
+  size_t smem = 0;
+  int cap_ne = 0, cap_p = 0, cap_halo = 0;
+  void* block = nullptr;      // the allocation of all that follows
+  unsigned long long* words = nullptr;
+  unsigned* epoch = nullptr;
+  unsigned long long* z = nullptr;
+  size_t words_bytes = 0;     // with the epoch and z
+  void* cta = nullptr;
+  int* halo = nullptr;
+  unsigned short* slot = nullptr;
+};
+
 // Device mirror of one Matrix_Type plus the Krylov workspace of its solves.
 struct tf_matrix_s {
   tf_ctx_s* ctx = nullptr;
@@ -138,6 +154,7 @@ struct tf_matrix_s {
   int spmv_grid = 1;
   int vec_grid = 1;
   int vec_dir = 0;       // walking direction of the vector kernels (see tf_fp64.cu)
+  tf_resident_s res;
   // ICC level schedule (built at registration for diagonal-first matrices)
   int icc_ready = 0;
   int* d_levf_rows = nullptr;  // forward-sweep rows grouped by level
@@ -186,7 +203,9 @@ struct tf_matrix_s {
 // Multi-RHS drop-in (tf_fp64.cu): slice allocation and the solve on
 // device-resident val / x_i / b_i (x and b slices of nt doubles each).
 int tf_fp64_run_multi(tf_matrix_s* m, int prec, int nrhs);
-int tf_slices_ensure(tf_matrix_s* m, int nrhs);   // allocate slices 1..nrhs-1
+// Slices 1..nrhs-1; states_only: their solve states alone (what resident
+// solves on the caller's arrays need).
+int tf_slices_ensure(tf_matrix_s* m, int nrhs, bool states_only = false);
 void tf_slices_free(tf_matrix_s* m);
 
 // FP64 drop-in entry points implemented in tf_fp64.cu
@@ -205,9 +224,17 @@ int tf_fp64_residual(tf_matrix_s* m, const double* val, const double* b,
                      const double* x, double* r);
 int tf_fp64_nrms(tf_matrix_s* m, const double* val, const double* r,
                  const double* x, int has_norm, double norm, double* out);
+int tf_resident_build(tf_matrix_s* m, const int* row0);
+size_t tf_resident_bytes(int n, int64_t nnz);
+int tf_resident_run(tf_matrix_s* m, int prec, const tf::SolveParams* p, double* x, double* b,
+                    tf::SolveState* st, int write_val);
+int tf_resident_reset(tf_matrix_s* m);
+// Whether Jacobi / none solves of m run as one resident kernel.
+bool tf_resident(const tf_matrix_s* m);
 int tf_icc_build(tf_matrix_s* m, const int* h_row0, const int* h_col0);
 int tf_icc_prepare(tf_matrix_s* m);   // before a solve with ICC
 void tf_icc_free(tf_matrix_s* m);
+size_t tf_icc_bytes(int n, int64_t nnz);   // the records of both sweeps, for budgeting
 tf::IccResid tf_icc_resid(const tf_matrix_s* m);
 // Registration behind tf_matrix_register; want_icc = 0 skips the ICC level
 // schedule.  Device bytes the matrix will hold, for budgeting.

@@ -654,3 +654,36 @@ def test_icc_sweeps_at_their_edges(gpu_ctx, case):
     n = len(a[4])
     args = (*a, np.zeros(n), "cg", "icc", 300, 1e-10, 1.0)
     check_parity(gpu_solve(gpu_ctx, *args), oracle_solve(*args), 1e-10, exact_iters=True)
+
+
+@pytest.mark.parametrize("prec,norm", [("jacobi", 1.0), ("none", None)])
+@pytest.mark.parametrize("case", ["1", "255", "257", "37889-rows", "75777-rows", "wide-band",
+                                  "halo-too-large", "largest-hex", "too-large-hex"])
+def test_resident_solve_at_its_edges(gpu_ctx, case, prec, norm):
+    """The one-kernel solve of matrices that fit the chip where its shapes
+    change -- one row, one row more than a CTA's, one more than 148 CTAs of 256
+    or 512 rows, rows of 41 entries, a halo that does not fit (every row
+    refers to rows of all CTAs), the largest hex that fits and one that does
+    not -- against the oracle after a few iterations."""
+    from tflows_b200.grids import hex_grid
+    if case.endswith("hex"):
+        g = hex_grid(*((67, 66, 68) if case == "largest-hex" else (75, 74, 76)))
+        s = systems.pressure_system(g, 3, tol=1e-10, miter=9)
+        a = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b)
+    elif case == "wide-band":
+        a = _band_system(3000, list(range(1, 21)), 8)
+    elif case == "halo-too-large":
+        a = _band_system(60000, [1] + list(range(1000, 60000, 2500)), 9)
+    else:
+        n = int(case.split("-")[0])
+        a = _band_system(n, [o for o in (1, 31, 900) if o < n], 10)
+    n = len(a[4])
+    x0 = np.random.default_rng(4).uniform(-0.5, 0.5, n)
+    args = (*a, x0, "cg", prec, 9, 1e-300, norm)
+    g, o = gpu_solve(gpu_ctx, *args), oracle_solve(*args)
+    assert g[3] == o[3] and rel_l2(g[0], o[0]) <= 1e-12
+    # The recursive residual after 9 steps: its rounding, about 9 eps |x0|-sized
+    # terms a row, is 1e-13 of the first residual; on one row it is all rounding.
+    assert g[4] == pytest.approx(o[4], rel=1e-9, abs=1e-12 * n)
+    assert np.allclose(g[1], o[1], rtol=4e-16, atol=0)
+    assert np.allclose(g[2], o[2], rtol=4e-16, atol=0)
