@@ -386,8 +386,8 @@ int tf_pool_cancel(tf_pool p, int64_t req);
 /* Resident structures: requests reusing a held registration (`reused`),
  * registrations currently held and their budgeted bytes.  A request whose
  * row/col/dia arrays (same addresses, same sampled contents, same sizes)
- * were registered by an earlier request runs on that registration when the
- * worker holding it takes it.  No reference counterpart. */
+ * were registered by an earlier request runs on that registration when no
+ * other request is using it.  No reference counterpart. */
 int tf_pool_resident(tf_pool p, long long* reused, int* held, size_t* held_bytes);
 int tf_pool_destroy(tf_pool p);
 

@@ -22,15 +22,19 @@
 // (Create_Native.f90 builds it once; every outer iteration only refills
 // val and b).  A registered matrix therefore stays on the device after its
 // request, keyed by the caller's row/col/dia pointers, sizes and a sampled
-// fingerprint of their contents; a later request with the same key, taken
-// by the worker that holds it, skips validation, tiling, renumbering and
-// the structure upload.  Held structures count toward the budget and are
-// released, least recently used first, when a new request needs the room.
-// A worker looks a few requests down the queue for one whose structure it
-// holds before taking the head.
+// fingerprint of their contents; a later request with the same key skips
+// validation, tiling, renumbering and the structure upload, whichever worker
+// takes it: an idle held structure moves to that worker's context (its last
+// solve has been waited for, so nothing on the other stream refers to it).
+// Held per worker, a stream of requests over 24 meshes on 8 workers registered
+// half of them again and again.  Held structures count toward the budget and
+// are released, least recently used first, when a new request needs the room.
+// A worker looks a few requests down the queue for one whose structure is
+// held and idle before taking the head.
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -86,7 +90,7 @@ uint64_t structure_key(int n, int64_t nnz, const int* row, const int* col, const
   return h;
 }
 
-constexpr int kLookahead = 16;   // queued requests a worker scans for its own structures
+constexpr int kLookahead = 16;   // queued requests a worker scans for a held structure
 }  // namespace
 
 struct tf_pool_s {
@@ -106,7 +110,6 @@ struct tf_pool_s {
   struct Held {
     uint64_t key = 0;
     tf_matrix_s* m = nullptr;
-    int owner = 0;
     bool in_use = false;
     size_t bytes = 0;
     uint64_t last = 0;
@@ -114,10 +117,19 @@ struct tf_pool_s {
   std::vector<Held> held;
   uint64_t tick = 0;
 
-  int find_held(uint64_t key, int w) const {
+  int find_held(uint64_t key) const {
     for (size_t i = 0; i < held.size(); ++i)
-      if (held[i].key == key && held[i].owner == w && !held[i].in_use) return (int)i;
+      if (held[i].key == key && !held[i].in_use) return (int)i;
     return -1;
+  }
+  // m's next solve runs on ctx: its stream and its lent pinned state.
+  static void adopt(tf_matrix_s* m, tf_ctx_s* ctx) {
+    m->ctx = ctx;
+    if (m->host_lent) {
+      m->h_state = ctx->h_state;
+      m->h_params = ctx->h_params;
+    }
+    if (m->ren) adopt(m->ren, ctx);
   }
   // Release idle held structures, least recently used first, until `need`
   // more bytes fit in the budget.  Caller holds mu.
@@ -127,19 +139,19 @@ struct tf_pool_s {
       for (size_t i = 0; i < held.size(); ++i)
         if (!held[i].in_use && (victim < 0 || held[i].last < held[victim].last)) victim = (int)i;
       if (victim < 0) return false;
-      tf_matrix_free(held[victim].m);   // stream-ordered on its owner's stream
+      tf_matrix_free(held[victim].m);   // on its last worker's stream
       used -= held[victim].bytes;
       held.erase(held.begin() + victim);
     }
     return true;
   }
-  // Pick worker w's next request: one whose structure it holds among the
-  // first kLookahead, else the head if it fits.  Caller holds mu.
-  std::shared_ptr<PoolReq> pick(int w, int* slot) {
+  // Pick a worker's next request: one whose structure is held and idle among
+  // the first kLookahead, else the head if it fits.  Caller holds mu.
+  std::shared_ptr<PoolReq> pick(int* slot) {
     *slot = -1;
     const int look = std::min<int>((int)queue.size(), kLookahead);
     for (int q = 0; q < look; ++q) {
-      const int h = find_held(queue[q]->key, w);
+      const int h = find_held(queue[q]->key);
       if (h >= 0) {
         auto r = queue[q];
         queue.erase(queue.begin() + q);
@@ -197,13 +209,14 @@ struct tf_pool_s {
         std::unique_lock<std::mutex> lk(mu);
         cv_work.wait(lk, [&] {
           if (stop) return true;
-          r = pick(w, &h);
+          r = pick(&h);
           return r != nullptr;
         });
         if (stop) return;
         if (h >= 0) {
           held[h].in_use = true;
           m = held[h].m;
+          adopt(m, ctx);
           ++reused;
         } else {
           used += r->bytes;
@@ -225,7 +238,6 @@ struct tf_pool_s {
           Held e;
           e.key = r->key;
           e.m = m;
-          e.owner = w;
           e.bytes = r->bytes;
           e.last = ++tick;
           held.push_back(e);
@@ -313,6 +325,11 @@ extern "C" int tf_pool_submit(tf_pool p, int solver, int prec, int n, int64_t nn
   r->t_submit = Clock::now();
   p->live[r->id] = r;
   ++p->submitted;
+  // What the resident solve or the ICC sweeps keep besides (a request that
+  // the matrix and its vectors leave room for is not refused over these).
+  if (r->bytes <= p->budget)
+    r->bytes = std::min(p->budget, r->bytes + (prec == TF_PREC_ICC ? tf_icc_bytes(n, nnz)
+                                                                    : tf_resident_bytes(n, nnz)));
   if (r->bytes > p->budget) {      // can never be admitted
     r->status = TF_ERR_OOM;
     r->done = true;
