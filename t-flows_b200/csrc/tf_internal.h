@@ -185,14 +185,18 @@ struct tf_matrix_s {
   int* d_perm = nullptr;
   int* d_src = nullptr;
   tf_matrix_s* active = nullptr;  // the matrix the last solve ran on
-  // Face topology for device-side assembly (tf_assemble.cu): per face the
-  // two cells (0-based, -1 on a boundary) and pos(1:2) (0-based entries),
-  // per cell its faces in ascending order (bit 0: the cell is the face's c2).
+  // Face topology for device-side assembly (tf_assemble.cu).  d_cf_other
+  // set: per 32 cells the lists of AsmLists (d_cf_ptr, d_cf the faces).
+  // Otherwise per face the two cells (0-based, -1 on a boundary) and pos(1:2)
+  // (0-based entries), per cell its faces in ascending order (bit 0: the cell
+  // is the face's c2).
   int n_faces = 0;
   int* d_face_cell = nullptr;
   int* d_face_pos = nullptr;
   int* d_cf_ptr = nullptr;
   int* d_cf = nullptr;
+  int* d_cf_other = nullptr;
+  unsigned short* d_cf_entry = nullptr;
   // Multi-RHS solves: slices for right-hand sides 2..kMaxRhs (allocated on
   // first use), pinned states of all right-hand sides, cached graphs per
   // (rhs count, preconditioner, x update deferred).

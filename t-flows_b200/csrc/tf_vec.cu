@@ -19,16 +19,57 @@ struct VecRed {
   double* out;
 };
 
+// The kernels walk the entries in pairs, kPairs pairs of every array loaded
+// before the first is used.  Pair j is entries 2 j and 2 j + 1: one 16-byte
+// access when every array allows it (VEC), two of 8 bytes otherwise -- the same
+// entries in the same thread either way, so sums do not depend on alignment.
+constexpr int kPairs = 4;
+
+template <bool VEC>
+__device__ __forceinline__ double2 get2(const double* x, int j) {
+  if (VEC) return reinterpret_cast<const double2*>(x)[j];
+  return make_double2(x[2 * j], x[2 * j + 1]);
+}
+template <bool VEC>
+__device__ __forceinline__ void put2(double* x, int j, double2 v) {
+  if (VEC) {
+    reinterpret_cast<double2*>(x)[j] = v;
+  } else {
+    x[2 * j] = v.x;
+    x[2 * j + 1] = v.y;
+  }
+}
+
 // y = a x + b y (Cg.f90:166-170 p = z + beta p, :204-209 x + alfa p and
 // r - alfa q); first: y = a x; a == 0: y = b y.
+template <bool VEC>
 __global__ void __launch_bounds__(kVecThreads) k_vec_axpby(int n, double a, const double* x,
                                                            double b, double* y, int first) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    if (first) y[i] = __dmul_rn(a, x[i]);
-    else if (a == 0.0) y[i] = __dmul_rn(b, y[i]);
-    else y[i] = __dadd_rn(__dmul_rn(a, x[i]), __dmul_rn(b, y[i]));
+  const int np = n >> 1, stride = gridDim.x * blockDim.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  auto one = [&](double xi, double yi) {
+    if (first) return __dmul_rn(a, xi);
+    if (a == 0.0) return __dmul_rn(b, yi);
+    return __dadd_rn(__dmul_rn(a, xi), __dmul_rn(b, yi));
+  };
+  for (int j0 = t; j0 < np; j0 += kPairs * stride) {
+    double2 xv[kPairs], yv[kPairs];
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) {
+      const int j = j0 + u * stride;
+      xv[u] = yv[u] = make_double2(0.0, 0.0);
+      if (j < np) {
+        if (first || a != 0.0) xv[u] = get2<VEC>(x, j);
+        if (!first) yv[u] = get2<VEC>(y, j);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) {
+      const int j = j0 + u * stride;
+      if (j < np) put2<VEC>(y, j, make_double2(one(xv[u].x, yv[u].x), one(xv[u].y, yv[u].y)));
+    }
   }
+  if ((n & 1) && t == 0) y[n - 1] = one(x[n - 1], first ? 0.0 : y[n - 1]);
 }
 
 __global__ void __launch_bounds__(kVecThreads) k_vec_gather(int n, const double* src,
@@ -53,26 +94,51 @@ __global__ void __launch_bounds__(kVecThreads) k_vec_recip(int n, const double* 
 // KIND 0: sum a_i b_i (b null: sum a_i); 1: sum r_i^2 / d_i^2
 // (Normalized_Root_Mean_Square.f90:33-36); 2: z = r d_inv (Prec_Solve.f90:
 // 44-49) and sum z_i r_i (Cg.f90:151-155); 3: min and max of x.
-template <int KIND>
+template <int KIND, bool VEC>
 __global__ void __launch_bounds__(kVecThreads) k_vec_reduce(int n, const double* a,
                                                             const double* b, double* z,
                                                             VecRed red) {
   __shared__ double scratch[2 * (kVecThreads / 32)];
   double s0 = KIND == 3 ? red_identity<kMin>() : 0.0;
   double s1 = red_identity<kMax>();
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    if (KIND == 0) s0 = __dadd_rn(s0, b ? __dmul_rn(a[i], b[i]) : a[i]);
-    if (KIND == 1) s0 = __dadd_rn(s0, nrms_term(a[i], b[i]));
+  auto one = [&](double ai, double bi) -> double {   // returns z
+    if (KIND == 0) s0 = __dadd_rn(s0, b ? __dmul_rn(ai, bi) : ai);
+    if (KIND == 1) s0 = __dadd_rn(s0, nrms_term(ai, bi));
     if (KIND == 2) {
-      const double zi = __dmul_rn(a[i], b[i]);
-      z[i] = zi;
-      s0 = __dadd_rn(s0, __dmul_rn(zi, a[i]));
+      const double zi = __dmul_rn(ai, bi);
+      s0 = __dadd_rn(s0, __dmul_rn(zi, ai));
+      return zi;
     }
     if (KIND == 3) {
-      s0 = fmin(s0, a[i]);
-      s1 = fmax(s1, a[i]);
+      s0 = fmin(s0, ai);
+      s1 = fmax(s1, ai);
     }
+    return 0.0;
+  };
+  const int np = n >> 1, stride = gridDim.x * blockDim.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int j0 = t; j0 < np; j0 += kPairs * stride) {
+    double2 av[kPairs], bv[kPairs];
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) {
+      const int j = j0 + u * stride;
+      if (j < np) {
+        av[u] = get2<VEC>(a, j);
+        bv[u] = b ? get2<VEC>(b, j) : make_double2(0.0, 0.0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) {
+      const int j = j0 + u * stride;
+      if (j < np) {
+        const double zx = one(av[u].x, bv[u].x), zy = one(av[u].y, bv[u].y);
+        if (KIND == 2) put2<VEC>(z, j, make_double2(zx, zy));
+      }
+    }
+  }
+  if ((n & 1) && t == 0) {
+    const double zi = one(a[n - 1], b ? b[n - 1] : 0.0);
+    if (KIND == 2) z[n - 1] = zi;
   }
   if (KIND == 3) {
     double v[2] = {block_red<kMin>(s0, scratch), block_red<kMax>(s1, scratch)};
@@ -97,8 +163,13 @@ namespace {
 
 constexpr int kVecMaxBlocks = 1024;
 
+// Whether 16-byte accesses are allowed on all of the arrays (null: none).
+bool pairs_aligned(const void* x, const void* y, const void* z = nullptr) {
+  return (((uintptr_t)x | (uintptr_t)y | (uintptr_t)z) & 15) == 0;
+}
+
 int vec_grid(tf_ctx_s* c, int n) {
-  return std::max(1, std::min({(n + kVecThreads - 1) / kVecThreads, c->sm_count * 4,
+  return std::max(1, std::min({(n + kVecThreads - 1) / kVecThreads, c->sm_count * 8,
                                kVecMaxBlocks}));
 }
 
@@ -125,7 +196,12 @@ int vec_reduce(tf_ctx ctx, int n, const double* a, const double* b, double* z, d
   VecRed red;
   int st = vec_scratch(ctx, &red, out);
   if (st != TF_OK) return st;
-  k_vec_reduce<KIND><<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, a, b, z, red);
+  // a whole batch of pairs a thread where there is that much
+  const int grid = vec_grid(ctx, (n + 2 * kPairs - 1) / (2 * kPairs));
+  if (pairs_aligned(a, b, z))
+    k_vec_reduce<KIND, true><<<grid, kVecThreads, 0, ctx->stream>>>(n, a, b, z, red);
+  else
+    k_vec_reduce<KIND, false><<<grid, kVecThreads, 0, ctx->stream>>>(n, a, b, z, red);
   TF_CUDA_TRY(cudaGetLastError());
   return TF_OK;
 }
@@ -138,7 +214,11 @@ extern "C" int tf_vec_axpby(tf_ctx ctx, int n, double a, const double* d_x, doub
   if (!ctx || n < 0 || (n > 0 && (!d_x || !d_y))) return TF_ERR_ARG;
   if (n == 0) return TF_OK;
   TF_CUDA_TRY(cudaSetDevice(ctx->device));
-  k_vec_axpby<<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, a, d_x, b, d_y, first);
+  const int grid = vec_grid(ctx, (n + 2 * kPairs - 1) / (2 * kPairs));
+  if (pairs_aligned(d_x, d_y))
+    k_vec_axpby<true><<<grid, kVecThreads, 0, ctx->stream>>>(n, a, d_x, b, d_y, first);
+  else
+    k_vec_axpby<false><<<grid, kVecThreads, 0, ctx->stream>>>(n, a, d_x, b, d_y, first);
   TF_CUDA_TRY(cudaGetLastError());
   return TF_OK;
   TF_API_END

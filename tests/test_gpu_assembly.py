@@ -93,3 +93,42 @@ def test_device_momentum_assembly_is_bitwise_and_solves_alike(gpu_ctx, kind):
         assert (it1, r1) == (it2, r2) and np.array_equal(x1, x2)
     finally:
         m.close()
+
+
+@pytest.mark.parametrize("case", ["one-cell-wide", "tiles", "long-row", "foreign-pos"])
+def test_row_assembly_at_its_edges(gpu_ctx, case):
+    """The cell-by-cell assembly where it can go wrong: one cell more than a
+    tile of 128, a cell with more faces than a tile in shared memory holds
+    entries, and a pos map that leaves the cells' own rows (assembled face by
+    face): bit for bit the loop restatement."""
+    torch = _torch()
+    if case == "long-row":   # a hub cell joined to 5,000 others
+        n = 5001
+        faces = np.stack([np.ones(n - 1), np.arange(2, n + 1)], axis=1).astype(np.int32)
+        g = grids.Grid(n_cells=n, faces_c=faces, sx=np.ones(n - 1), sy=np.zeros(n - 1),
+                       sz=np.zeros(n - 1), dx=np.linspace(1, 2, n - 1), dy=np.zeros(n - 1),
+                       dz=np.zeros(n - 1), fw=np.linspace(0.1, 0.9, n - 1), vol=np.ones(n),
+                       h_min=1.0, h_mean=1.0, kind="hub", meta={})
+    else:
+        dims = {"one-cell-wide": (1, 1, 129), "tiles": (16, 8, 3), "foreign-pos": (4, 3, 2)}[case]
+        g = grids.hex_grid(*dims)
+    c = systems.create_matrix(g)
+    fc = systems.face_coef(g)
+    pos = c.pos.copy()
+    inner = np.nonzero(g.interior)[0]
+    if case == "foreign-pos":   # the entries of two faces exchanged
+        pos[inner[0]], pos[inner[-1]] = c.pos[inner[-1]], c.pos[inner[0]]
+    vm = np.random.default_rng(5).uniform(0.5, 2.0, g.n_cells)
+    want = O.assemble_pressure(g, pos, c.dia, c.nnz, fc, np.zeros(g.n_faces, bool), v_m=vm)
+    m = native.Matrix(gpu_ctx, c.row, c.col, c.dia)
+    try:
+        native.faces_register(gpu_ctx, m, g.faces_c, pos)
+        d = [torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (fc, g.fw, vm)]
+        dval = torch.full((c.nnz,), 7.0, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        native.assemble_pressure(gpu_ctx, m, d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(),
+                                 0, dval.data_ptr())
+        gpu_ctx.sync()
+        assert np.array_equal(_bits(dval.cpu().numpy()), _bits(want))
+    finally:
+        m.close()
