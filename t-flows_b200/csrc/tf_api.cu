@@ -173,17 +173,15 @@ int dev_alloc(tf_ctx_s* ctx, T** p, size_t count) {
 
 }  // namespace
 
-// Zeroed device memory; stream-ordered on the context's stream when the
-// context asks for it (no device-wide synchronisation).
+// Device memory, zeroed on the context's stream (which does not wait for the
+// legacy stream: a cudaMemset there could run after the stream's own writes);
+// stream-ordered too when the context asks for it (no device-wide
+// synchronisation).
 int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes) {
   *p = nullptr;
-  if (ctx->async_alloc) {
-    TF_CUDA_TRY(cudaMallocAsync(p, bytes, ctx->stream));
-    TF_CUDA_TRY(cudaMemsetAsync(*p, 0, bytes, ctx->stream));
-  } else {
-    TF_CUDA_TRY(cudaMalloc(p, bytes));
-    TF_CUDA_TRY(cudaMemset(*p, 0, bytes));
-  }
+  if (ctx->async_alloc) TF_CUDA_TRY(cudaMallocAsync(p, bytes, ctx->stream));
+  else TF_CUDA_TRY(cudaMalloc(p, bytes));
+  TF_CUDA_TRY(cudaMemsetAsync(*p, 0, bytes, ctx->stream));
   return TF_OK;
 }
 

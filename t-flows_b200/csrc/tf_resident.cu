@@ -178,7 +178,7 @@ __device__ __forceinline__ bool res_exchange(const ResArgs& a, double (&v)[NV], 
 // (30^3) 20.6 / 5.4, 130,000 21.9 / 6.5, 300,000 25.6 / 10.7, 21,000
 // polyhedral cells 19.2 / 5.9; a solve's fixed part 105 / 70 us.
 template <int PREC, bool NORM, int RPT, int T>
-__global__ void __launch_bounds__(T, T * RPT <= 512 ? 2 : 1) k_resident(ResArgs a) {
+__global__ void __launch_bounds__(T, 1) k_resident(ResArgs a) {
   extern __shared__ __align__(16) unsigned char tf_res_smem[];
   __shared__ ResShared<T> sh;
   double* sval = reinterpret_cast<double*>(tf_res_smem);
