@@ -154,7 +154,8 @@ int tf_solve_native(tf_ctx ctx, tf_matrix m, const char* solver,
  * two result scalars.  When all three are 16-byte aligned (as cudaMalloc'd
  * arrays are) the solve runs on them in place: the first call with a new
  * set of arrays builds the solve's CUDA graph on them, later calls with the
- * same arrays reuse it.  val is then read in 16-byte units, so up to 8
+ * same arrays reuse it (a Jacobi or unpreconditioned solve of a matrix that
+ * fits the chip is one kernel and needs no graph).  val is then read in 16-byte units, so up to 8
  * bytes past its last entry are read (inside any cudaMalloc allocation).
  * Arrays off a 16-byte boundary are copied into the matrix's own buffers
  * and back (same results). */
@@ -191,7 +192,10 @@ int tf_last_history(tf_ctx ctx, double* hist, int cap, int* count);
  * 2 s): a streaming kernel of the solve (the SpMV and residual passes) stops
  * at its first wait for a tile's copies or a free pipeline stage after this
  * much time since its start -- or once such a wait has been blocked that
- * long -- and the solve ends with TF_ERR_TIMEOUT.  Before a stopped CTA
+ * long -- and the solve ends with TF_ERR_TIMEOUT.  The one-kernel solve of a
+ * matrix that fits the chip stops when an exchange between its CTAs is not
+ * complete this long after the one before it, and so do the waits of the ICC
+ * sweeps.  Before a stopped CTA
  * exits it still waits for the copies it started (with the default limit),
  * and the context stays usable.  The reference has no counterpart (its
  * failures stop the run, Shared/Message_Mod/Error.f90:74). */

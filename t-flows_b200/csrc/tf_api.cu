@@ -182,6 +182,7 @@ int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes) {
   if (ctx->async_alloc) TF_CUDA_TRY(cudaMallocAsync(p, bytes, ctx->stream));
   else TF_CUDA_TRY(cudaMalloc(p, bytes));
   TF_CUDA_TRY(cudaMemsetAsync(*p, 0, bytes, ctx->stream));
+  if (!ctx->async_alloc) TF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return TF_OK;
 }
 

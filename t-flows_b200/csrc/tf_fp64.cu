@@ -365,6 +365,7 @@ struct SpArgs {
   int nrows;
   VecArgs v;
   double* out_scalar;  // building-block mode: receives the dot product
+  double* pq;          // ... and so does this, unless null
 };
 
 // Rows through shared-memory tiles (CFG < kTileNone; PAT: row-pattern
@@ -529,6 +530,7 @@ __global__ void __launch_bounds__(cfg_threads<CFG, PAT>(), cfg_min_blocks<CFG, P
   unsigned* cnt = st ? &st->counter[kCntSpmv] : reinterpret_cast<unsigned*>(a.out_scalar + 1);
   if (grid_reduce_last<1>(v, ops, a.v.part, cnt, scratch) && threadIdx.x == 0) {
     if (a.out_scalar) a.out_scalar[0] = v[0];
+    if (a.pq) *a.pq = v[0];
     if (st) {
       st->pq = v[0];
       st->alpha = __ddiv_rn(st->rho, v[0]);
@@ -735,6 +737,7 @@ SpArgs make_sp_args(tf_matrix_s* m, const VecArgs& v) {
   s.nrows = m->ni;
   s.v = v;
   s.out_scalar = nullptr;
+  s.pq = nullptr;
   return s;
 }
 
@@ -1109,7 +1112,7 @@ int tf_fp64_run(tf_matrix_s* m, int prec) {
 namespace {
 template <int CFG, int PAT>
 int launch_spmv(tf_matrix_s* m, const double* val, const double* p, double* q,
-                double* scal) {
+                double* scal, double* pq) {
   VecArgs va = make_vec_args(m);
   va.st = nullptr;
   va.p = const_cast<double*>(p);
@@ -1117,6 +1120,7 @@ int launch_spmv(tf_matrix_s* m, const double* val, const double* p, double* q,
   SpArgs sa = make_sp_args(m, va);
   sa.val = val;
   sa.out_scalar = scal;
+  sa.pq = pq;
   k_spmv_alpha<CFG, PAT><<<m->spmv_grid, cfg_threads<CFG, PAT>(), cfg_smem<CFG, PAT>(),
                           m->ctx->stream>>>(sa);
   TF_CUDA_TRY(cudaGetLastError());
@@ -1147,13 +1151,9 @@ static double* bb_scalar(tf_matrix_s* m) { return m->d_part + 8 * kMaxBlocks; }
 int tf_fp64_spmv(tf_matrix_s* m, const double* val, const double* p, double* q,
                  double* pq) {
   double* scal = bb_scalar(m);
-  const int st = dispatch_cfg(m->tile_cfg, m->npat > 0, [&](auto C, auto P) {
-    return launch_spmv<decltype(C)::value, decltype(P)::value>(m, val, p, q, scal);
+  return dispatch_cfg(m->tile_cfg, m->npat > 0, [&](auto C, auto P) {
+    return launch_spmv<decltype(C)::value, decltype(P)::value>(m, val, p, q, scal, pq);
   });
-  if (st == TF_OK && pq)
-    TF_CUDA_TRY(cudaMemcpyAsync(pq, scal, sizeof(double), cudaMemcpyDeviceToDevice,
-                                m->ctx->stream));
-  return st;
 }
 
 int tf_fp64_residual(tf_matrix_s* m, const double* val, const double* b,
