@@ -353,10 +353,12 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, unsigned parit
     if (*abort_flag || globaltimer_ns() > deadline) return false;
   return globaltimer_ns() <= deadline;
 }
-// A deadline that costs a clock register to look at: the global timer is read
-// at the first look and then only when kLookCycles have passed since, so a
-// limit is kept to within that (the one-CTA ICC sweeps took 3 % longer with the
-// timer read at every wait).
+// A deadline whose looks mostly read the SM clock only: the global timer is read
+// at the first look after the limit starts to count and then only when
+// kLookCycles have passed since, so a limit is kept to within that (the one-CTA
+// ICC sweeps took 3 % longer with the timer read at every wait).  Once passed it
+// stays so until renewed: a wait that gave up early may leave it to the next
+// look to end the kernel.
 struct Deadline {
   unsigned long long limit, ns;   // globaltimer
   long long look;                 // SM clock at which to read it again
@@ -371,8 +373,14 @@ struct Deadline {
   __device__ __forceinline__ bool passed() {
     const long long c = clock64();
     if (c < look) return false;
+    if (globaltimer_ns() > ns) return true;   // and again at the next look
     look = c + kLookCycles;
-    return globaltimer_ns() > ns;
+    return false;
+  }
+  // Passed, from now on (globaltimer is past 0).
+  __device__ __forceinline__ void give_up() {
+    ns = 0;
+    look = 0;
   }
 };
 // mbar_wait_or_abort on such a deadline.

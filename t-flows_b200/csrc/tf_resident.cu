@@ -327,12 +327,15 @@ __global__ void __launch_bounds__(T, 1) k_resident(ResArgs a) {
       if (h < nh) sp[nr + h] = direction(zh[u], sp[nr + h]);
     }
     // The rest of a large halo: exchange 2 has seen every CTA's sums, which
-    // were sent after its z, so a few polls at most.
+    // were sent after its z, so a few polls at most.  A thread that gives up
+    // here goes on without its z to exchange 1, which then fails: its deadline
+    // stays passed.
     for (int h = t + kResAhead * T; h < nh; h += T) {
       double z = 0.0;
       bool gone = false;
-      for (int spin = 0; !take(h, z, tag) && !gone; ++spin)
-        if ((spin & 63) == 63) gone = deadline.passed();
+      for (int spin = 0; !gone && !take(h, z, tag); ++spin)
+        if ((spin & 63) == 63) gone = deadline.passed() || *(volatile int*)&a.st->status != 0;
+      if (gone) deadline.give_up();
       sp[nr + h] = direction(z, sp[nr + h]);
     }
 #pragma unroll

@@ -61,6 +61,57 @@ def test_wait_limit_runs_out_then_context_recovers(kind, monkeypatch):
         ctx.close()
 
 
+def wide_halo_system(n=30000):
+    """Symmetric and diagonally dominant; 256 consecutive rows refer to some 2,300
+    rows outside them, more than the four a thread polls for ahead."""
+    rng = np.random.default_rng(11)
+    offs = [1] + list(range(3000, 18000, 3000))
+    i = np.arange(n)
+    w = {o: -rng.uniform(0.2, 1.0, n) for o in offs}   # entry (i, i + o)
+    r = np.concatenate([np.concatenate([i[:n - o], i[o:]]) for o in offs])
+    c = np.concatenate([np.concatenate([i[o:], i[:n - o]]) for o in offs])
+    v = np.concatenate([np.concatenate([w[o][:n - o]] * 2) for o in offs])
+    diag = 0.3 - np.bincount(r, weights=v, minlength=n)
+    r, c, v = (np.concatenate([a, b]) for a, b in ((r, i), (c, i), (v, diag)))
+    order = np.lexsort((c, c != r, r))   # the diagonal first
+    row = np.zeros(n + 1, np.int32)
+    row[1:] = np.cumsum(np.bincount(r, minlength=n))
+    return row + 1, c[order].astype(np.int32) + 1, row[:-1] + 1, v[order], rng.uniform(-1, 1, n)
+
+
+def test_solve_under_a_short_limit_is_right_or_times_out():
+    """The one-kernel solve over wait limits around the time of its exchanges:
+    a call that succeeds has the bits of an unhurried one, whatever waits were
+    close to their end, and one that does not leaves the context usable."""
+    row, col, dia, val, b = wide_halo_system()
+    ctx = native.Context(0)
+    m = native.Matrix(ctx, row, col, dia)
+    try:
+        def run():
+            v, x, bb = val.copy(), np.zeros(len(b)), b.copy()
+            return native.solve(ctx, m, "cg", "jacobi", v, x, bb, 30, 1e-300, 1.0), x
+
+        want, x0 = run()
+        assert want[0] == 30
+        ended = []
+        for limit in np.geomspace(1e-9, 1e-3, 60):
+            ctx.set_wait_limit(limit)
+            try:
+                got, x = run()
+                ended.append(True)
+                assert got == want and np.array_equal(x, x0)
+            except native.TFError as e:
+                assert e.status == 4
+                ended.append(False)
+        assert not ended[0] and ended[-1]
+        ctx.set_wait_limit(0.0)
+        got, x = run()
+        assert got == want and np.array_equal(x, x0)
+    finally:
+        m.close()
+        ctx.close()
+
+
 def test_wait_limit_argument_checks(gpu_ctx):
     with pytest.raises(native.TFError):
         gpu_ctx.set_wait_limit(-1.0)
