@@ -231,7 +231,7 @@ int tf_fp64_nrms(tf_matrix_s* m, const double* val, const double* r,
 int tf_resident_build(tf_matrix_s* m, const int* row0);
 size_t tf_resident_bytes(int n, int64_t nnz);
 int tf_resident_run(tf_matrix_s* m, int prec, const tf::SolveParams* p, double* x, double* b,
-                    tf::SolveState* st, int write_val);
+                    tf::SolveState* st, const tf::SolveState* before, int write_val);
 int tf_resident_reset(tf_matrix_s* m);
 // Whether Jacobi / none solves of m run as one resident kernel.
 bool tf_resident(const tf_matrix_s* m);

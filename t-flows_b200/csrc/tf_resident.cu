@@ -57,6 +57,7 @@ struct ResArgs {
   unsigned long long* words;     // [2][CTAs][kResWords]
   unsigned* epoch;               // number of the last exchange on these words
   SolveState* st;
+  const SolveState* before;      // of the solve before this one on the same words, or null
   double tol, norm;
   int miter, hist_cap;
   double* hist;
@@ -190,6 +191,12 @@ __global__ void __launch_bounds__(T, 1) k_resident(ResArgs a) {
   const ResCta me = a.cta[blockIdx.x];
   const int r0 = me.r0, nr = me.r1 - me.r0, j0 = a.row[r0], ne = a.row[me.r1] - j0, nh = me.nh;
   SolveState* st = a.st;
+  // The right-hand side before this one gave up: its words carry numbers this
+  // solve would use again, so nothing is solved until the host has reset them.
+  if (a.before && a.before->status != 0) {
+    if (blockIdx.x == 0 && t == 0) st->status = a.before->status;
+    return;
+  }
   unsigned tag = *a.epoch;
   Deadline deadline(a.wait_ns ? a.wait_ns : kWaitLimitNs);
 
@@ -576,9 +583,10 @@ bool tf_resident(const tf_matrix_s* m) {
 }
 
 // One solve on val, x, b (device) with the parameters in *p, on m's stream;
-// the state goes to *st.  write_val: val is scaled back into place.
+// the state goes to *st.  before: the state of the solve launched before it, when
+// the host has not looked at that yet.  write_val: val is scaled back into place.
 int tf_resident_run(tf_matrix_s* m, int prec, const SolveParams* p, double* x, double* b,
-                    SolveState* st, int write_val) {
+                    SolveState* st, const SolveState* before, int write_val) {
   ResArgs a{};
   a.n = m->ni;
   a.row = m->d_row;
@@ -592,6 +600,7 @@ int tf_resident_run(tf_matrix_s* m, int prec, const SolveParams* p, double* x, d
   a.slot = m->res.slot;
   a.words = m->res.words;
   a.st = st;
+  a.before = before;
   a.tol = p->tol;
   a.norm = p->norm;
   a.miter = p->miter;

@@ -112,6 +112,54 @@ def test_solve_under_a_short_limit_is_right_or_times_out():
         ctx.close()
 
 
+def test_right_hand_sides_after_one_that_timed_out_are_left_alone():
+    """Several right-hand sides on a matrix that fits the chip are solved one
+    after another on the caller's arrays.  Over wait limits around the time of
+    the first exchange (the first solve waits for its values, later ones find
+    them in L2): an x has changed only if every x before it is solved."""
+    import torch
+    row, col, dia, val, b = wide_halo_system()
+    n, nrhs = len(b), 3
+    B = np.stack([b, -0.5 * b[::-1], np.roll(b, 7)])
+    flush = torch.zeros(1 << 25, dtype=torch.float64, device="cuda")   # larger than L2
+    ctx = native.Context(0)
+    m = native.Matrix(ctx, row, col, dia)
+    try:
+        def run():
+            d = [torch.from_numpy(a).cuda() for a in (val, np.zeros((nrhs, n)), B)]
+            flush.add_(1.0)
+            torch.cuda.synchronize()
+            try:
+                r = native.solve_multi_device(ctx, m, "cg", "jacobi", nrhs,
+                                              *(t.data_ptr() for t in d), 5, 1e-300, 1.0)
+            except native.TFError as e:
+                assert e.status == 4
+                r = None
+            torch.cuda.synchronize()
+            return r, [t.cpu().numpy() for t in d]
+
+        want, (v0, x0, b0) = run()
+        assert want is not None
+        late = 0
+        for limit in np.concatenate([[1e-9], np.geomspace(1e-6, 3e-5, 80), [1e-3]]):
+            ctx.set_wait_limit(limit)
+            got, (v, x, bb) = run()
+            if got is not None:
+                assert got == want and np.array_equal(x, x0)
+                continue
+            late += 1
+            solved = [np.array_equal(x[i], x0[i]) for i in range(nrhs)]
+            for i in range(1, nrhs):
+                assert all(solved[:i]) or not x[i].any(), (limit, solved)
+        assert late > 0 and got == want
+        ctx.set_wait_limit(0.0)
+        got, (v, x, bb) = run()
+        assert got == want and all(np.array_equal(a, c) for a, c in ((v, v0), (x, x0), (bb, b0)))
+    finally:
+        m.close()
+        ctx.close()
+
+
 def test_wait_limit_argument_checks(gpu_ctx):
     with pytest.raises(native.TFError):
         gpu_ctx.set_wait_limit(-1.0)
