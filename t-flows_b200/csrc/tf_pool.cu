@@ -25,7 +25,8 @@
 // fingerprint of their contents; a later request with the same key skips
 // validation, tiling, renumbering and the structure upload, whichever worker
 // takes it: an idle held structure moves to that worker's context (its last
-// solve has been waited for, so nothing on the other stream refers to it).
+// request, failed ones too, has been waited for, so nothing on the other
+// stream refers to it).
 // Held per worker, a stream of requests over 24 meshes on 8 workers registered
 // half of them again and again.  Held structures count toward the budget and
 // are released, least recently used first, when a new request needs the room.
@@ -225,6 +226,8 @@ struct tf_pool_s {
         r->t_start = Clock::now();
       }
       const int st = tf_guarded([&] { return run(ctx, *r, &m); });
+      // another worker may take the structure next, on its own stream
+      if (st != TF_OK) cudaStreamSynchronize(ctx->stream);
       {
         std::lock_guard<std::mutex> lk(mu);
         if (h >= 0) {

@@ -620,7 +620,8 @@ int tf_resident_run(tf_matrix_s* m, int prec, const SolveParams* p, double* x, d
 }
 
 // After a solve that gave up: the words of unfinished exchanges and the
-// recorded status.
+// recorded status.  Waited for: the matrix's next solve may run on another
+// context's stream (tf_pool.cu).
 int tf_resident_reset(tf_matrix_s* m) {
   if (!m->res.ctas) return TF_OK;
   cudaStream_t s = m->ctx->stream;
@@ -628,5 +629,6 @@ int tf_resident_reset(tf_matrix_s* m) {
   TF_CUDA_TRY(cudaMemsetAsync(&m->d_state->status, 0, sizeof(int), s));
   for (auto* c : m->slices)
     if (c) TF_CUDA_TRY(cudaMemsetAsync(&c->d_state->status, 0, sizeof(int), s));
+  TF_CUDA_TRY(cudaStreamSynchronize(s));
   return TF_OK;
 }
