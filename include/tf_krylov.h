@@ -391,7 +391,8 @@ int tf_pool_cancel(tf_pool p, int64_t req);
  * registrations currently held and their budgeted bytes.  A request whose
  * row/col/dia arrays (same addresses, same sampled contents, same sizes)
  * were registered by an earlier request runs on that registration when no
- * other request is using it.  No reference counterpart. */
+ * other request is using it; up to 16 such requests are taken before the
+ * one at the head of the queue.  No reference counterpart. */
 int tf_pool_resident(tf_pool p, long long* reused, int* held, size_t* held_bytes);
 int tf_pool_destroy(tf_pool p);
 

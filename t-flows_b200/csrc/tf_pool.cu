@@ -31,7 +31,7 @@
 // half of them again and again.  Held structures count toward the budget and
 // are released, least recently used first, when a new request needs the room.
 // A worker looks a few requests down the queue for one whose structure is
-// held and idle before taking the head.
+// held and idle before taking the head, kPassLimit times at most for one head.
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -72,6 +72,7 @@ struct PoolReq {
   int niter = 0;
   double fin_res = 0.0;
   bool done = false;
+  int passed = 0;             // requests taken before it while it was the head
 };
 // Sampled fingerprint of a Matrix_Type structure plus the caller's array
 // addresses: equal keys mean "the same arrays, unchanged where sampled".
@@ -92,6 +93,10 @@ uint64_t structure_key(int n, int64_t nnz, const int* row, const int* col, const
 }
 
 constexpr int kLookahead = 16;   // queued requests a worker scans for a held structure
+// Requests taken before the head of the queue at most, as long as it is the
+// head: under steady traffic on held structures a request on a new one would
+// otherwise wait without bound.
+constexpr int kPassLimit = 16;
 }  // namespace
 
 struct tf_pool_s {
@@ -147,23 +152,26 @@ struct tf_pool_s {
     return true;
   }
   // Pick a worker's next request: one whose structure is held and idle among
-  // the first kLookahead, else the head if it fits.  Caller holds mu.
+  // the first kLookahead, else (or once kPassLimit went before it) the head if
+  // it fits.  Caller holds mu.
   std::shared_ptr<PoolReq> pick(int* slot) {
     *slot = -1;
-    const int look = std::min<int>((int)queue.size(), kLookahead);
+    if (queue.empty()) return nullptr;
+    const auto head = queue.front();
+    const int look = head->passed < kPassLimit ? std::min<int>((int)queue.size(), kLookahead) : 1;
     for (int q = 0; q < look; ++q) {
       const int h = find_held(queue[q]->key);
       if (h >= 0) {
         auto r = queue[q];
+        if (q > 0) ++head->passed;
         queue.erase(queue.begin() + q);
         *slot = h;
         return r;
       }
     }
-    if (queue.empty() || !make_room(queue.front()->bytes)) return nullptr;
-    auto r = queue.front();
+    if (!make_room(head->bytes)) return nullptr;
     queue.pop_front();
-    return r;
+    return head;
   }
 
   // Run one request on worker w's context, on matrix m when it is held.

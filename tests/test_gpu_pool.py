@@ -150,3 +150,26 @@ def test_pool_cancel_queued_request(gpu_ctx):
         assert r["niter"] == want[1] and np.array_equal(r["x"], want[0])
     finally:
         p.close()
+
+
+def test_pool_request_on_a_new_structure_is_not_passed_over_for_good(gpu_ctx):
+    """300 queued requests on a held structure and one on a new structure ahead
+    of them: the worker takes at most 16 of them before it."""
+    known = systems.small_hex(16, seed=8, kind="pressure", ratio=1.02)
+    new = systems.small_hex(11, seed=9, kind="pressure")
+    want = _reference(gpu_ctx, new)
+    p = pool.Pool(workers=1, mem_budget=1 << 30)
+    try:
+        p.wait(p.submit(known))                 # held from here on
+        busy = [p.submit(known, tol=0.0, miter=20000) for _ in range(2)]
+        first = p.submit(new)
+        rest = [p.submit(known, tol=0.0, miter=500) for _ in range(300)]
+        r = p.wait(first)
+        done = p.stats()["completed"]
+        assert r["niter"] == want[1] and np.array_equal(r["x"], want[0])
+        # itself, the 3 before it, the 16, and what ran until wait() returned
+        assert done <= 120, done
+        for rid in busy + rest:
+            p.wait(rid)
+    finally:
+        p.close()
