@@ -201,6 +201,11 @@ int tf_last_history(tf_ctx ctx, double* hist, int cap, int* count);
  * failures stop the run, Shared/Message_Mod/Error.f90:74). */
 int tf_ctx_set_wait_limit(tf_ctx ctx, double seconds);
 
+/* For tests of failure paths: of the matrix and workspace allocations this
+ * context makes from now on, `skip` succeed and the `count` after them fail
+ * with TF_ERR_OOM without asking the device (0, 0: none fail). */
+int tf_ctx_fail_allocs(tf_ctx ctx, int skip, int count);
+
 /* Pin (page-lock) a host array the caller will pass to tf_solve on every
  * call, e.g. A % val, so its copies run at full PCIe/C2C bandwidth.
  * Wraps cudaHostRegister / cudaHostUnregister. */

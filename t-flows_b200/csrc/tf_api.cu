@@ -132,6 +132,15 @@ extern "C" int tf_ctx_set_wait_limit(tf_ctx ctx, double seconds) {
   TF_API_END
 }
 
+extern "C" int tf_ctx_fail_allocs(tf_ctx ctx, int skip, int count) {
+  TF_API_BEGIN
+  if (!ctx || skip < 0 || count < 0) return TF_ERR_ARG;
+  ctx->alloc_skip = skip;
+  ctx->alloc_fail = count;
+  return TF_OK;
+  TF_API_END
+}
+
 extern "C" int tf_last_history(tf_ctx ctx, double* hist, int cap, int* count) {
   TF_API_BEGIN
   if (!ctx || !count || (cap > 0 && !hist)) return TF_ERR_ARG;
@@ -179,6 +188,11 @@ int dev_alloc(tf_ctx_s* ctx, T** p, size_t count) {
 // synchronisation).
 int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes) {
   *p = nullptr;
+  if (ctx->alloc_fail > 0 && ctx->alloc_skip-- <= 0) {   // tf_ctx_fail_allocs
+    ctx->alloc_skip = 0;
+    --ctx->alloc_fail;
+    return TF_ERR_OOM;
+  }
   if (ctx->async_alloc) TF_CUDA_TRY(cudaMallocAsync(p, bytes, ctx->stream));
   else TF_CUDA_TRY(cudaMalloc(p, bytes));
   TF_CUDA_TRY(cudaMemsetAsync(*p, 0, bytes, ctx->stream));

@@ -54,6 +54,7 @@ __device__ __forceinline__ double p_coef(const double* fc, const double* fw, con
 constexpr int kAsmCells = 128;
 constexpr int kAsmBatch = 6;        // a hex cell's faces
 constexpr int kAsmEntries = 4096;   // largest tile kept in shared memory
+constexpr int kAsmPlaces = 1 << 20; // places of the lists that are always granted
 
 // Visit v of lane t of the slice of cells 32 s .. 32 s + 31 is at ptr[s] +
 // 32 v + t: face | flags, or -1; its other cell; its entry, counted from the
@@ -279,6 +280,82 @@ struct AsmMomentum {
 
 using namespace tf;
 
+namespace {
+
+void faces_free(tf_matrix_s* m) {
+  for (int** p : {&m->d_face_cell, &m->d_face_pos, &m->d_cf_ptr, &m->d_cf, &m->d_cf_other}) {
+    tf_dev_free(m->ctx, *p);
+    *p = nullptr;
+  }
+  tf_dev_free(m->ctx, m->d_cf_entry);
+  m->d_cf_entry = nullptr;
+  m->n_faces = 0;
+}
+
+template <class T>
+int dev_copy(tf_ctx_s* ctx, T** d, const std::vector<T>& h) {
+  const int st = tf_dev_alloc_bytes(ctx, (void**)d, h.size() * sizeof(T));
+  if (st != TF_OK) return st;
+  TF_CUDA_TRY(cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice,
+                              ctx->stream));
+  return TF_OK;
+}
+
+// The lists of the assembly by rows; sptr: where the slices of 32 cells
+// start, rows: the row pointers.
+int row_lists(tf_matrix_s* m, int n_faces, const int* faces_c, const int* pos,
+              const std::vector<int>& sptr, const std::vector<int>& rows) {
+  std::vector<int> face((size_t)sptr.back() + 32, -1), other(face.size()), fill(m->nt, 0);
+  std::vector<unsigned short> entry(face.size());
+  for (int s = 0; s < n_faces; ++s) {   // every cell's faces in ascending order
+    const int c2 = faces_c[2 * s + 1];
+    for (int k = 0; k < (c2 > 0 ? 2 : 1); ++k) {
+      const int c = faces_c[2 * s + k] - 1;
+      const size_t at = (size_t)sptr[c >> 5] + 32 * (size_t)fill[c]++ + (c & 31);
+      face[at] = s | (k ? kAsmSecond : 0) | (c2 > 0 ? 0 : kAsmBoundary);
+      if (c2 <= 0) continue;
+      other[at] = faces_c[2 * s + 1 - k] - 1;
+      entry[at] = (unsigned short)(pos[2 * s + k] - 1 - rows[c]);
+    }
+  }
+  int st = dev_copy(m->ctx, &m->d_cf_ptr, sptr);
+  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf, face);
+  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf_other, other);
+  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf_entry, entry);
+  TF_CUDA_TRY(cudaStreamSynchronize(m->ctx->stream));
+  return st;
+}
+
+// The lists of the assembly face by face.
+int face_lists(tf_matrix_s* m, int n_faces, const int* faces_c, const int* pos,
+               const std::vector<int>& cnt) {
+  const int n = m->nt;
+  std::vector<int> fcell((size_t)2 * n_faces + 2), fpos((size_t)2 * n_faces + 2);
+  for (int s = 0; s < n_faces; ++s) {
+    const int c2 = faces_c[2 * s + 1];
+    fcell[2 * s] = faces_c[2 * s] - 1;
+    fcell[2 * s + 1] = c2 > 0 ? c2 - 1 : -1;
+    fpos[2 * s] = c2 > 0 ? pos[2 * s] - 1 : -1;
+    fpos[2 * s + 1] = c2 > 0 ? pos[2 * s + 1] - 1 : -1;
+  }
+  // cell -> faces in ascending face order; bit 0: the cell is the face's c2
+  std::vector<int> ptr((size_t)n + 1, 0);
+  for (int c = 0; c < n; ++c) ptr[c + 1] = ptr[c] + cnt[c];
+  std::vector<int> cf((size_t)ptr[n] + 1), fill(ptr.begin(), ptr.end() - 1);
+  for (int s = 0; s < n_faces; ++s) {
+    cf[fill[fcell[2 * s]]++] = s << 1;
+    if (fcell[2 * s + 1] >= 0) cf[fill[fcell[2 * s + 1]]++] = (s << 1) | 1;
+  }
+  int st = dev_copy(m->ctx, &m->d_face_cell, fcell);
+  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_face_pos, fpos);
+  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf_ptr, ptr);
+  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf, cf);
+  TF_CUDA_TRY(cudaStreamSynchronize(m->ctx->stream));
+  return st;
+}
+
+}  // namespace
+
 extern "C" int tf_faces_register(tf_ctx ctx, tf_matrix m, int n_faces, const int* faces_c,
                                  const int* pos) {
   TF_API_BEGIN
@@ -298,12 +375,7 @@ extern "C" int tf_faces_register(tf_ctx ctx, tf_matrix m, int n_faces, const int
   }
   std::lock_guard<std::mutex> lk(m->mu);
   TF_CUDA_TRY(cudaSetDevice(ctx->device));
-  for (void* p : {(void*)m->d_face_cell, (void*)m->d_face_pos, (void*)m->d_cf_ptr,
-                  (void*)m->d_cf, (void*)m->d_cf_other, (void*)m->d_cf_entry})
-    if (p) cudaFree(p);
-  m->d_face_cell = m->d_face_pos = m->d_cf_ptr = m->d_cf = m->d_cf_other = nullptr;
-  m->d_cf_entry = nullptr;
-  m->n_faces = 0;
+  faces_free(m);
   // Every entry in its own cell's row (as Create_Matrix builds pos): the rows
   // are assembled cell by cell.
   std::vector<int> rows((size_t)n + 1);
@@ -317,80 +389,32 @@ extern "C" int tf_faces_register(tf_ctx ctx, tf_matrix m, int n_faces, const int
         const int c = faces_c[2 * s + k] - 1, p = pos[2 * s + k] - 1;
         own = own && p >= rows[c] && p < rows[c + 1];
       }
-  if (own) {
-    const int slices = (n + 31) / 32;
-    std::vector<int> sptr((size_t)slices + 1, 0), fill(n, 0);
-    for (int s = 0; s < slices; ++s) {
-      int w = 0;
-      for (int c = 32 * s; c < std::min(n, 32 * s + 32); ++c) w = std::max(w, cnt[c]);
-      if ((long long)sptr[s] + 32LL * w > INT_MAX) return TF_ERR_OOM;
-      sptr[s + 1] = sptr[s] + 32 * w;
+  // Lists padded to the longest of 32 cells: not where a few cells with many
+  // faces would make them several times the faces (10 bytes a place).
+  std::vector<int> sptr((size_t)(n + 31) / 32 + 1, 0);
+  long long places = 0, visits = 0;
+  for (int c0 = 0; c0 < n && own; c0 += 32) {
+    int w = 0;
+    for (int c = c0; c < std::min(n, c0 + 32); ++c) {
+      w = std::max(w, cnt[c]);
+      visits += cnt[c];
     }
-    std::vector<int> face((size_t)sptr[slices] + 32, -1), other(face.size());
-    std::vector<unsigned short> entry(face.size());
-    for (int s = 0; s < n_faces; ++s) {   // every cell's faces in ascending order
-      const int c2 = faces_c[2 * s + 1];
-      for (int k = 0; k < (c2 > 0 ? 2 : 1); ++k) {
-        const int c = faces_c[2 * s + k] - 1;
-        const size_t at = (size_t)sptr[c >> 5] + 32 * (size_t)fill[c]++ + (c & 31);
-        face[at] = s | (k ? kAsmSecond : 0) | (c2 > 0 ? 0 : kAsmBoundary);
-        if (c2 <= 0) continue;
-        other[at] = faces_c[2 * s + 1 - k] - 1;
-        entry[at] = (unsigned short)(pos[2 * s + k] - 1 - rows[c]);
-      }
-    }
-    int st = tf_dev_alloc_bytes(ctx, (void**)&m->d_cf_ptr, sptr.size() * sizeof(int));
-    if (st == TF_OK) st = tf_dev_alloc_bytes(ctx, (void**)&m->d_cf, face.size() * sizeof(int));
-    if (st == TF_OK)
-      st = tf_dev_alloc_bytes(ctx, (void**)&m->d_cf_other, other.size() * sizeof(int));
-    if (st == TF_OK) st = tf_dev_alloc_bytes(ctx, (void**)&m->d_cf_entry, entry.size() * 2);
-    if (st != TF_OK) return st;
-    cudaStream_t s = ctx->stream;
-    TF_CUDA_TRY(cudaMemcpyAsync(m->d_cf_ptr, sptr.data(), sptr.size() * sizeof(int),
-                                cudaMemcpyHostToDevice, s));
-    TF_CUDA_TRY(cudaMemcpyAsync(m->d_cf, face.data(), face.size() * sizeof(int),
-                                cudaMemcpyHostToDevice, s));
-    TF_CUDA_TRY(cudaMemcpyAsync(m->d_cf_other, other.data(), other.size() * sizeof(int),
-                                cudaMemcpyHostToDevice, s));
-    TF_CUDA_TRY(cudaMemcpyAsync(m->d_cf_entry, entry.data(), entry.size() * 2,
-                                cudaMemcpyHostToDevice, s));
-    TF_CUDA_TRY(cudaStreamSynchronize(s));
-    m->n_faces = n_faces;
-    return TF_OK;
+    places += 32LL * w;
+    own = places <= INT_MAX - 32;
+    if (own) sptr[c0 / 32 + 1] = (int)places;
   }
-  std::vector<int> fcell((size_t)2 * n_faces + 2), fpos((size_t)2 * n_faces + 2);
-  for (int s = 0; s < n_faces; ++s) {
-    const int c2 = faces_c[2 * s + 1];
-    fcell[2 * s] = faces_c[2 * s] - 1;
-    fcell[2 * s + 1] = c2 > 0 ? c2 - 1 : -1;
-    fpos[2 * s] = c2 > 0 ? pos[2 * s] - 1 : -1;
-    fpos[2 * s + 1] = c2 > 0 ? pos[2 * s + 1] - 1 : -1;
+  own = own && places <= std::max(4 * visits, (long long)kAsmPlaces);
+  int st = TF_ERR_OOM;
+  if (own) st = row_lists(m, n_faces, faces_c, pos, sptr, rows);
+  if (st == TF_ERR_OOM) {   // too long, or no room for them
+    faces_free(m);
+    cudaGetLastError();
+    st = face_lists(m, n_faces, faces_c, pos, cnt);
   }
-  // cell -> faces in ascending face order; bit 0: the cell is the face's c2
-  std::vector<int> ptr((size_t)n + 1, 0);
-  for (int c = 0; c < n; ++c) ptr[c + 1] = ptr[c] + cnt[c];
-  std::vector<int> cf((size_t)ptr[n] + 1), fill(ptr.begin(), ptr.end() - 1);
-  for (int s = 0; s < n_faces; ++s) {
-    cf[fill[fcell[2 * s]]++] = s << 1;
-    if (fcell[2 * s + 1] >= 0) cf[fill[fcell[2 * s + 1]]++] = (s << 1) | 1;
-  }
-  int st = tf_dev_alloc_bytes(ctx, (void**)&m->d_face_cell, fcell.size() * sizeof(int));
-  if (st == TF_OK) st = tf_dev_alloc_bytes(ctx, (void**)&m->d_face_pos, fpos.size() * sizeof(int));
-  if (st == TF_OK) st = tf_dev_alloc_bytes(ctx, (void**)&m->d_cf_ptr, ptr.size() * sizeof(int));
-  if (st == TF_OK) st = tf_dev_alloc_bytes(ctx, (void**)&m->d_cf, cf.size() * sizeof(int));
-  if (st != TF_OK) return st;
-  cudaStream_t s = ctx->stream;
-  TF_CUDA_TRY(cudaMemcpyAsync(m->d_face_cell, fcell.data(), fcell.size() * sizeof(int),
-                              cudaMemcpyHostToDevice, s));
-  TF_CUDA_TRY(cudaMemcpyAsync(m->d_face_pos, fpos.data(), fpos.size() * sizeof(int),
-                              cudaMemcpyHostToDevice, s));
-  TF_CUDA_TRY(cudaMemcpyAsync(m->d_cf_ptr, ptr.data(), ptr.size() * sizeof(int),
-                              cudaMemcpyHostToDevice, s));
-  TF_CUDA_TRY(cudaMemcpyAsync(m->d_cf, cf.data(), cf.size() * sizeof(int),
-                              cudaMemcpyHostToDevice, s));
-  TF_CUDA_TRY(cudaStreamSynchronize(s));
-  m->n_faces = n_faces;
-  return TF_OK;
+  // Half a list is none: tf_assemble_* refuses the matrix.
+  if (st != TF_OK) faces_free(m);
+  else m->n_faces = n_faces;
+  return st;
   TF_API_END
 }
 

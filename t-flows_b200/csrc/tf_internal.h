@@ -60,6 +60,7 @@ struct tf_ctx_s {
   cudaStream_t stream = nullptr;
   int history = 0;
   unsigned long long wait_ns = 0;   // bounded-wait limit of this context's solves (0: default)
+  int alloc_skip = 0, alloc_fail = 0;   // allocations to grant, then to fail (tests)
   double* d_vec_scratch = nullptr;  // partial sums of the tf_vec_* reductions (tf_vec.cu)
   std::vector<double> last_hist;
   int last_count = 0;

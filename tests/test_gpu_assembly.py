@@ -132,3 +132,56 @@ def test_row_assembly_at_its_edges(gpu_ctx, case):
         assert np.array_equal(_bits(dval.cpu().numpy()), _bits(want))
     finally:
         m.close()
+
+
+@pytest.mark.parametrize("case", ["no-room", "hub"])
+def test_faces_without_room_for_the_row_lists(gpu_ctx, case):
+    """Lists that find no room, or that one cell with 40,000 faces would pad to
+    32 times the faces, give way to the assembly face by face, bit for bit;
+    where that finds no room either, nothing half-registered is left behind."""
+    torch = _torch()
+    n = 40001 if case == "hub" else 300
+    nf = n - 1
+    faces = np.stack([np.ones(nf), np.arange(2, n + 1)], axis=1).astype(np.int32)
+    if case == "no-room":
+        faces[:, 0] = np.arange(1, n)
+    one = np.ones(nf)
+    g = grids.Grid(n_cells=n, faces_c=faces, sx=one, sy=0 * one, sz=0 * one,
+                   dx=np.linspace(1, 2, nf), dy=0 * one, dz=0 * one,
+                   fw=np.linspace(0.1, 0.9, nf), vol=np.ones(n), h_min=1.0, h_mean=1.0,
+                   kind=case, meta={})
+    c = systems.create_matrix(g)
+    fc = systems.face_coef(g)
+    vm = np.random.default_rng(6).uniform(0.5, 2.0, n)
+    want = O.assemble_pressure(g, c.pos, c.dia, c.nnz, fc, np.zeros(nf, bool), v_m=vm)
+    d = [torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (fc, g.fw, vm)]
+    dval = torch.full((c.nnz,), 7.0, dtype=torch.float64, device="cuda")
+    m = native.Matrix(gpu_ctx, c.row, c.col, c.dia)
+
+    def assemble():
+        dval.fill_(7.0)
+        torch.cuda.synchronize()
+        native.assemble_pressure(gpu_ctx, m, d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(),
+                                 0, dval.data_ptr())
+        gpu_ctx.sync()
+        return _bits(dval.cpu().numpy())
+
+    try:
+        for skip in range(4):
+            gpu_ctx.fail_allocs(skip, 1 if case == "no-room" else 0)
+            native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
+            assert np.array_equal(assemble(), _bits(want))
+        for skip in range(4):   # of the row lists' and then of the others' four
+            gpu_ctx.fail_allocs(skip, 5)
+            with pytest.raises(native.TFError) as e:
+                native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
+            assert e.value.status == 2
+            with pytest.raises(native.TFError) as e:
+                assemble()
+            assert e.value.status == 3
+        gpu_ctx.fail_allocs(0, 0)
+        native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
+        assert np.array_equal(assemble(), _bits(want))
+    finally:
+        gpu_ctx.fail_allocs(0, 0)
+        m.close()
