@@ -220,8 +220,7 @@ void tf_matrix_free(tf_matrix_s* m) {
                   m->d_hist, m->d_state, m->d_params, m->d_levf_rows, m->d_levb_rows,
                   m->d_icc_d, m->d_icc_dinv,
                   m->d_pat, m->d_pat_tab, m->d_perm, m->d_src,
-                  m->d_face_cell, m->d_face_pos, m->d_cf_ptr, m->d_cf, m->d_cf_other,
-                  m->d_cf_entry, m->res.block};
+                  m->face_block, m->res.block};
   for (void* p : ptrs) tf_dev_free(m->ctx, p);
   tf_icc_free(m);
   if (!m->host_lent) {

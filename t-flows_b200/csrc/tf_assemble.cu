@@ -20,6 +20,7 @@
 #include <limits.h>
 
 #include <algorithm>
+#include <memory>
 #include <vector>
 
 #include "tf_internal.h"
@@ -126,6 +127,38 @@ __global__ void __launch_bounds__(kAsmCells, 10) k_asm_rows(int n, const int* __
   if (!staged) return;
   __syncthreads();
   for (int e = t; e < ne; e += kAsmCells) val[j0 + e] = tile[e];
+}
+
+// Whether every entry of pos (1-based) lies in the row of its face's cell.
+__global__ void __launch_bounds__(256) k_asm_own(int nf, const int* __restrict__ faces,
+                                                 const int* __restrict__ pos,
+                                                 const int* __restrict__ row, int* foreign) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nf; s += gridDim.x * blockDim.x) {
+    if (faces[2 * s + 1] <= 0) continue;
+    for (int k = 0; k < 2; ++k) {
+      const int c = faces[2 * s + k] - 1, p = pos[2 * s + k] - 1;
+      if (p < row[c] || p >= row[c + 1]) *foreign = 1;
+    }
+  }
+}
+
+// The other cells and the entries of the listed faces, a thread a cell.
+__global__ void __launch_bounds__(256) k_asm_lists(int n, const int* __restrict__ faces,
+                                                   const int* __restrict__ pos,
+                                                   const int* __restrict__ row,
+                                                   const int* __restrict__ ptr,
+                                                   const int* __restrict__ face, int* other,
+                                                   unsigned short* entry) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  for (int v = ptr[c >> 5] + (c & 31); v < ptr[(c >> 5) + 1]; v += 32) {
+    const int f = face[v];
+    if (f < 0) break;
+    if (f & kAsmBoundary) continue;
+    const int s = f & kAsmFace, k = f & kAsmSecond ? 1 : 0;
+    other[v] = faces[2 * s + 1 - k] - 1;
+    entry[v] = (unsigned short)(pos[2 * s + k] - 1 - row[c]);
+  }
 }
 
 // Pressure: interior faces (Rhie_And_Chow.f90:183-205), then the open
@@ -283,46 +316,109 @@ using namespace tf;
 namespace {
 
 void faces_free(tf_matrix_s* m) {
-  for (int** p : {&m->d_face_cell, &m->d_face_pos, &m->d_cf_ptr, &m->d_cf, &m->d_cf_other}) {
-    tf_dev_free(m->ctx, *p);
-    *p = nullptr;
-  }
-  tf_dev_free(m->ctx, m->d_cf_entry);
+  tf_dev_free(m->ctx, m->face_block);
+  m->face_block = nullptr;
+  m->d_face_cell = m->d_face_pos = m->d_cf_ptr = m->d_cf = m->d_cf_other = nullptr;
   m->d_cf_entry = nullptr;
   m->n_faces = 0;
 }
 
+size_t place_bytes(size_t count, size_t size) { return (count * size + 127) & ~(size_t)127; }
+
+// Cuts `count` T off the block at p.
 template <class T>
-int dev_copy(tf_ctx_s* ctx, T** d, const std::vector<T>& h) {
-  const int st = tf_dev_alloc_bytes(ctx, (void**)d, h.size() * sizeof(T));
-  if (st != TF_OK) return st;
-  TF_CUDA_TRY(cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice,
-                              ctx->stream));
+T* cut(unsigned char*& p, size_t count) {
+  T* t = reinterpret_cast<T*>(p);
+  p += place_bytes(count, sizeof(T));
+  return t;
+}
+
+int upload(tf_ctx_s* ctx, int* d, const int* h, size_t count) {
+  if (count > 0)
+    TF_CUDA_TRY(cudaMemcpyAsync(d, h, count * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   return TF_OK;
 }
 
-// The lists of the assembly by rows; sptr: where the slices of 32 cells
-// start, rows: the row pointers.
+// The lists of the assembly by rows; cnt: faces a cell.  TF_ERR_OOM when there
+// is no room for them, *took = 0 when they are not for these faces.
 int row_lists(tf_matrix_s* m, int n_faces, const int* faces_c, const int* pos,
-              const std::vector<int>& sptr, const std::vector<int>& rows) {
-  std::vector<int> face((size_t)sptr.back() + 32, -1), other(face.size()), fill(m->nt, 0);
-  std::vector<unsigned short> entry(face.size());
-  for (int s = 0; s < n_faces; ++s) {   // every cell's faces in ascending order
-    const int c2 = faces_c[2 * s + 1];
-    for (int k = 0; k < (c2 > 0 ? 2 : 1); ++k) {
-      const int c = faces_c[2 * s + k] - 1;
-      const size_t at = (size_t)sptr[c >> 5] + 32 * (size_t)fill[c]++ + (c & 31);
-      face[at] = s | (k ? kAsmSecond : 0) | (c2 > 0 ? 0 : kAsmBoundary);
-      if (c2 <= 0) continue;
-      other[at] = faces_c[2 * s + 1 - k] - 1;
-      entry[at] = (unsigned short)(pos[2 * s + k] - 1 - rows[c]);
+              const std::vector<int>& cnt, int* took) {
+  const int n = m->nt;
+  *took = 0;
+  if (n_faces >= kAsmBoundary || m->max_row_len > 65536) return TF_OK;
+  // Padded to the longest of 32 cells: not where a few cells with many faces
+  // would make them several times the faces (10 bytes a place).
+  std::vector<int> sptr((size_t)(n + 31) / 32 + 1, 0);
+  long long places = 0, visits = 0;
+  for (int c0 = 0; c0 < n; c0 += 32) {
+    int w = 0;
+    for (int c = c0; c < std::min(n, c0 + 32); ++c) {
+      w = std::max(w, cnt[c]);
+      visits += cnt[c];
     }
+    places += 32LL * w;
+    if (places > INT_MAX - 32) return TF_OK;
+    sptr[c0 / 32 + 1] = (int)places;
   }
-  int st = dev_copy(m->ctx, &m->d_cf_ptr, sptr);
-  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf, face);
-  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf_other, other);
-  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf_entry, entry);
-  TF_CUDA_TRY(cudaStreamSynchronize(m->ctx->stream));
+  if (places > std::max(4 * visits, (long long)kAsmPlaces)) return TF_OK;
+  // Every cell's faces in ascending order, next[c]: the place of its next one.
+  std::unique_ptr<int[]> face(new int[places + 32]);
+  std::vector<int> next(n);
+  for (int c = 0; c < n; ++c) next[c] = sptr[c >> 5] + (c & 31);
+  auto put = [&](int c, int f) {
+    face[next[c]] = f;
+    next[c] += 32;
+  };
+  for (int s = 0; s < n_faces; ++s) {
+    const int c2 = faces_c[2 * s + 1];
+    put(faces_c[2 * s] - 1, s | (c2 > 0 ? 0 : kAsmBoundary));
+    if (c2 > 0) put(c2 - 1, s | kAsmSecond);
+  }
+  for (int c = 0; c < n; ++c)
+    for (int v = next[c]; v < sptr[(c >> 5) + 1]; v += 32) face[v] = -1;
+  // The rest is looked up on the device.
+  tf_ctx_s* ctx = m->ctx;
+  cudaStream_t s = ctx->stream;
+  const size_t words = (size_t)2 * n_faces, np = (size_t)places + 32;
+  // A flag, the faces, pos: in the values' workspace, which holds nothing between
+  // solves, unless boundary faces make them longer (an allocation and its
+  // release are a third of the call on 27,000 cells).
+  int *own = nullptr, *given = reinterpret_cast<int*>(m->d_val), foreign = 0;
+  auto build = [&]() -> int {
+    int st = TF_OK;
+    if (1 + 2 * words > (size_t)m->nnz * 2) {
+      st = tf_dev_alloc_bytes(ctx, (void**)&own, (1 + 2 * words) * sizeof(int));
+      given = own;
+    }
+    if (st == TF_OK)
+      st = tf_dev_alloc_bytes(ctx, &m->face_block, place_bytes(sptr.size(), 4) +
+                                                       2 * place_bytes(np, 4) + place_bytes(np, 2));
+    if (st != TF_OK) return st;
+    unsigned char* p = static_cast<unsigned char*>(m->face_block);
+    m->d_cf_ptr = cut<int>(p, sptr.size());
+    m->d_cf = cut<int>(p, np);
+    m->d_cf_other = cut<int>(p, np);
+    m->d_cf_entry = cut<unsigned short>(p, np);
+    int *d_faces = given + 1, *d_pos = d_faces + words;
+    TF_CUDA_TRY(cudaMemsetAsync(given, 0, sizeof(int), s));
+    st = upload(ctx, d_faces, faces_c, words);
+    if (st == TF_OK) st = upload(ctx, d_pos, pos, words);
+    if (st == TF_OK) st = upload(ctx, m->d_cf_ptr, sptr.data(), sptr.size());
+    if (st == TF_OK) st = upload(ctx, m->d_cf, face.get(), (size_t)places);
+    if (st != TF_OK) return st;
+    k_asm_own<<<ctx->sm_count * 8, 256, 0, s>>>(n_faces, d_faces, d_pos, m->d_row, given);
+    k_asm_lists<<<std::max(1, (n + 255) / 256), 256, 0, s>>>(n, d_faces, d_pos, m->d_row,
+                                                             m->d_cf_ptr, m->d_cf,
+                                                             m->d_cf_other, m->d_cf_entry);
+    TF_CUDA_TRY(cudaGetLastError());
+    TF_CUDA_TRY(cudaMemcpyAsync(&foreign, given, sizeof(int), cudaMemcpyDeviceToHost, s));
+    return TF_OK;
+  };
+  int st = build();
+  const cudaError_t e = cudaStreamSynchronize(s);   // the arrays copied from are still here
+  tf_dev_free(ctx, own);
+  if (st == TF_OK) TF_CUDA_TRY(e);
+  *took = !foreign;
   return st;
 }
 
@@ -346,10 +442,19 @@ int face_lists(tf_matrix_s* m, int n_faces, const int* faces_c, const int* pos,
     cf[fill[fcell[2 * s]]++] = s << 1;
     if (fcell[2 * s + 1] >= 0) cf[fill[fcell[2 * s + 1]]++] = (s << 1) | 1;
   }
-  int st = dev_copy(m->ctx, &m->d_face_cell, fcell);
-  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_face_pos, fpos);
-  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf_ptr, ptr);
-  if (st == TF_OK) st = dev_copy(m->ctx, &m->d_cf, cf);
+  int st = tf_dev_alloc_bytes(m->ctx, &m->face_block,
+                              place_bytes(fcell.size(), 4) + place_bytes(fpos.size(), 4) +
+                                  place_bytes(ptr.size(), 4) + place_bytes(cf.size(), 4));
+  if (st != TF_OK) return st;
+  unsigned char* p = static_cast<unsigned char*>(m->face_block);
+  m->d_face_cell = cut<int>(p, fcell.size());
+  m->d_face_pos = cut<int>(p, fpos.size());
+  m->d_cf_ptr = cut<int>(p, ptr.size());
+  m->d_cf = cut<int>(p, cf.size());
+  st = upload(m->ctx, m->d_face_cell, fcell.data(), fcell.size());
+  if (st == TF_OK) st = upload(m->ctx, m->d_face_pos, fpos.data(), fpos.size());
+  if (st == TF_OK) st = upload(m->ctx, m->d_cf_ptr, ptr.data(), ptr.size());
+  if (st == TF_OK) st = upload(m->ctx, m->d_cf, cf.data(), cf.size());
   TF_CUDA_TRY(cudaStreamSynchronize(m->ctx->stream));
   return st;
 }
@@ -378,35 +483,9 @@ extern "C" int tf_faces_register(tf_ctx ctx, tf_matrix m, int n_faces, const int
   faces_free(m);
   // Every entry in its own cell's row (as Create_Matrix builds pos): the rows
   // are assembled cell by cell.
-  std::vector<int> rows((size_t)n + 1);
-  TF_CUDA_TRY(cudaMemcpyAsync(rows.data(), m->d_row, rows.size() * sizeof(int),
-                              cudaMemcpyDeviceToHost, ctx->stream));
-  TF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  bool own = n_faces < kAsmBoundary && m->max_row_len <= 65536;
-  for (int s = 0; s < n_faces && own; ++s)
-    if (faces_c[2 * s + 1] > 0)
-      for (int k = 0; k < 2; ++k) {
-        const int c = faces_c[2 * s + k] - 1, p = pos[2 * s + k] - 1;
-        own = own && p >= rows[c] && p < rows[c + 1];
-      }
-  // Lists padded to the longest of 32 cells: not where a few cells with many
-  // faces would make them several times the faces (10 bytes a place).
-  std::vector<int> sptr((size_t)(n + 31) / 32 + 1, 0);
-  long long places = 0, visits = 0;
-  for (int c0 = 0; c0 < n && own; c0 += 32) {
-    int w = 0;
-    for (int c = c0; c < std::min(n, c0 + 32); ++c) {
-      w = std::max(w, cnt[c]);
-      visits += cnt[c];
-    }
-    places += 32LL * w;
-    own = places <= INT_MAX - 32;
-    if (own) sptr[c0 / 32 + 1] = (int)places;
-  }
-  own = own && places <= std::max(4 * visits, (long long)kAsmPlaces);
-  int st = TF_ERR_OOM;
-  if (own) st = row_lists(m, n_faces, faces_c, pos, sptr, rows);
-  if (st == TF_ERR_OOM) {   // too long, or no room for them
+  int took = 0;
+  int st = row_lists(m, n_faces, faces_c, pos, cnt, &took);
+  if (st == TF_ERR_OOM || (st == TF_OK && !took)) {
     faces_free(m);
     cudaGetLastError();
     st = face_lists(m, n_faces, faces_c, pos, cnt);

@@ -192,6 +192,7 @@ struct tf_matrix_s {
   // (0-based entries), per cell its faces in ascending order (bit 0: the cell
   // is the face's c2).
   int n_faces = 0;
+  void* face_block = nullptr;   // the allocation of all that follows
   int* d_face_cell = nullptr;
   int* d_face_pos = nullptr;
   int* d_cf_ptr = nullptr;

@@ -167,18 +167,16 @@ def test_faces_without_room_for_the_row_lists(gpu_ctx, case):
         return _bits(dval.cpu().numpy())
 
     try:
-        for skip in range(4):
-            gpu_ctx.fail_allocs(skip, 1 if case == "no-room" else 0)
+        gpu_ctx.fail_allocs(0, 1 if case == "no-room" else 0)   # the row lists'
+        native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
+        assert np.array_equal(assemble(), _bits(want))
+        gpu_ctx.fail_allocs(0, 2)                               # and the others'
+        with pytest.raises(native.TFError) as e:
             native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
-            assert np.array_equal(assemble(), _bits(want))
-        for skip in range(4):   # of the row lists' and then of the others' four
-            gpu_ctx.fail_allocs(skip, 5)
-            with pytest.raises(native.TFError) as e:
-                native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
-            assert e.value.status == 2
-            with pytest.raises(native.TFError) as e:
-                assemble()
-            assert e.value.status == 3
+        assert e.value.status == 2
+        with pytest.raises(native.TFError) as e:
+            assemble()
+        assert e.value.status == 3
         gpu_ctx.fail_allocs(0, 0)
         native.faces_register(gpu_ctx, m, g.faces_c, c.pos)
         assert np.array_equal(assemble(), _bits(want))
