@@ -182,10 +182,9 @@ int dev_alloc(tf_ctx_s* ctx, T** p, size_t count) {
 
 }  // namespace
 
-// Device memory, zeroed on the context's stream (which does not wait for the
-// legacy stream: a cudaMemset there could run after the stream's own writes);
-// stream-ordered too when the context asks for it (no device-wide
-// synchronisation).
+// Device memory, zeroed on the context's stream, where everything that uses it
+// runs too (cudaMemset's legacy stream would not be ordered with it), and
+// stream-ordered when the context asks for it (no device-wide synchronisation).
 int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes) {
   *p = nullptr;
   if (ctx->alloc_fail > 0 && ctx->alloc_skip-- <= 0) {   // tf_ctx_fail_allocs
@@ -196,7 +195,6 @@ int tf_dev_alloc_bytes(tf_ctx_s* ctx, void** p, size_t bytes) {
   if (ctx->async_alloc) TF_CUDA_TRY(cudaMallocAsync(p, bytes, ctx->stream));
   else TF_CUDA_TRY(cudaMalloc(p, bytes));
   TF_CUDA_TRY(cudaMemsetAsync(*p, 0, bytes, ctx->stream));
-  if (!ctx->async_alloc) TF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return TF_OK;
 }
 
