@@ -124,6 +124,11 @@ int tf_matrix_row_patterns(tf_matrix m);
  * entries in storage order, so row sums are unchanged).  0 otherwise.
  * No reference counterpart: a property of this library's device layout. */
 int tf_matrix_renumbered(tf_matrix m);
+/* CTAs of the one-kernel Jacobi / none solve of a matrix that fits the chip
+ * (of its renumbered copy when it has one); 0 before the first such solve,
+ * which lays it out, and for matrices that do not fit or have buffer cells.
+ * No reference counterpart. */
+int tf_matrix_resident(tf_matrix m);
 
 /* Solve A x = b.  Replaces Native_Type % Solve_Native (Solve_Native.f90:2-46)
  * and so Cg.f90:2-257 / Bicg.f90:2-269.  val, x and b are host arrays of

@@ -98,8 +98,10 @@ struct tf_icc_dir_s {
 };
 
 // The matrix's distribution over the CTAs of the resident solve
-// (tf_resident.cu); ctas = 0: it does not fit the chip.
+// (tf_resident.cu), made before the first Jacobi / none solve; rows = 0: it
+// does not fit the chip.
 struct tf_resident_s {
+  int rows = 0;               // rows a CTA
   int ctas = 0, shape = 0, threads = 0;
   size_t smem = 0;
   int cap_ne = 0, cap_p = 0, cap_halo = 0;
@@ -230,12 +232,13 @@ int tf_fp64_residual(tf_matrix_s* m, const double* val, const double* b,
                      const double* x, double* r);
 int tf_fp64_nrms(tf_matrix_s* m, const double* val, const double* r,
                  const double* x, int has_norm, double norm, double* out);
-int tf_resident_build(tf_matrix_s* m, const int* row0);
+void tf_resident_plan(tf_matrix_s* m, const int* row0);   // at registration
+int tf_resident_prepare(tf_matrix_s* m);   // before a solve without ICC
 size_t tf_resident_bytes(int n, int64_t nnz);
 int tf_resident_run(tf_matrix_s* m, int prec, const tf::SolveParams* p, double* x, double* b,
                     tf::SolveState* st, const tf::SolveState* before, int write_val);
 int tf_resident_reset(tf_matrix_s* m);
-// Whether Jacobi / none solves of m run as one resident kernel.
+// Whether Jacobi / none solves of m, once prepared, run as one resident kernel.
 bool tf_resident(const tf_matrix_s* m);
 int tf_icc_build(tf_matrix_s* m, const int* h_row0, const int* h_col0);
 int tf_icc_prepare(tf_matrix_s* m);   // before a solve with ICC

@@ -487,19 +487,20 @@ size_t res_smem(int ne, int p, int halo, int rows) {
   return (size_t)ne * 8 + (size_t)p * 8 + (size_t)halo * 4 + (size_t)ne * 2 +
          ((size_t)rows + 1) * 2 + 16;
 }
+// k_resident_build's shared memory: a bit a row, and the words' ranks.
+size_t res_bits(int n) { return (size_t)((n + 31) / 32) * 8; }
 constexpr size_t kResEpochBytes = 128;
 constexpr size_t kResSmemMax = 225 * 1024 - 2048;   // beside the exchange's static part
 
 }  // namespace
 
-// The rows of every CTA, their halos and the entries' places in p, when the
-// matrix fits the chip; otherwise m->res.ctas stays 0.  Made on the device
-// from its row and column arrays.
-int tf_resident_build(tf_matrix_s* m, const int* row0) {
+// Rows a CTA and the kernel's shape, when the matrix may fit the chip; otherwise
+// m->res.rows stays 0.  row0: its row pointers on the host.
+void tf_resident_plan(tf_matrix_s* m, const int* row0) {
   const int n = m->ni, sms = m->ctx->sm_count;
-  m->res.ctas = 0;
+  m->res.rows = 0;
   // (Buffer cells are rows that no CTA would own.)
-  if (n < 1 || m->nt != n) return TF_OK;
+  if (n < 1 || m->nt != n) return;
   // Rows a CTA: 256 (one a thread) while there are SMs for that many CTAs,
   // then as many as it takes (512 at the least: us an iteration at 27,000
   // rows 5.44 / 5.56 / 5.94 with 256 / 512 / 1024 rows a CTA).
@@ -508,19 +509,30 @@ int tf_resident_build(tf_matrix_s* m, const int* row0) {
   int shape = 0;
   while (shape < kResShapeCount && kResShapes[shape].rpt * kResShapes[shape].threads < rows)
     ++shape;
-  if (shape == kResShapeCount) return TF_OK;
+  if (shape == kResShapeCount) return;
   const int G = (n + rows - 1) / rows;
   int cap_ne = 0;
   for (int c = 0; c < G; ++c)
     cap_ne = std::max(cap_ne, row0[std::min(n, (c + 1) * rows)] - row0[c * rows]);
-  if (cap_ne > 65535 || res_smem(cap_ne, rows, 0, rows) > kResSmemMax) return TF_OK;
-  cap_ne = (cap_ne + 7) & ~7;   // keeps what follows aligned
-  const size_t bits = (size_t)((n + 31) / 32) * 8;   // words and their ranks
-  if (bits > kResSmemMax) return TF_OK;
+  if (cap_ne > 65535 || res_smem(cap_ne, rows, 0, rows) > kResSmemMax) return;
+  if (res_bits(n) > kResSmemMax) return;
+  m->res.rows = rows;
+  m->res.shape = shape;
+  m->res.cap_ne = (cap_ne + 7) & ~7;   // keeps what follows aligned
+}
+
+namespace {
+
+// The CTAs' halos and the entries' places in p, made on the device from the
+// matrix's row and column arrays; m->res.ctas stays 0 when they do not fit.
+int res_build(tf_matrix_s* m) {
+  const int n = m->ni, sms = m->ctx->sm_count, rows = m->res.rows, shape = m->res.shape;
+  const int G = (n + rows - 1) / rows, cap_ne = m->res.cap_ne;
+  const size_t bits = res_bits(n);
   cudaStream_t s = m->ctx->stream;
   TF_CUDA_TRY(cudaFuncSetAttribute(k_resident_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kResSmemMax));
-  int* d_largest = reinterpret_cast<int*>(m->d_part);   // zero between kernels' uses
+  int* d_largest = reinterpret_cast<int*>(m->d_part);   // free between kernels
   int largest = 0;
   TF_CUDA_TRY(cudaMemsetAsync(d_largest, 0, sizeof(int), s));
   k_resident_build<<<G, 512, bits, s>>>(m->d_row, m->d_col, n, rows, 0, nullptr, nullptr, nullptr,
@@ -561,17 +573,26 @@ int tf_resident_build(tf_matrix_s* m, const int* row0) {
                                         reinterpret_cast<ResCta*>(m->res.cta), m->res.halo,
                                         m->res.slot, nullptr);
   TF_CUDA_TRY(cudaGetLastError());
-  m->res.shape = shape;
   m->res.threads = kResShapes[shape].threads;
   m->res.smem = smem;
-  m->res.cap_ne = cap_ne;
   m->res.cap_p = cap_p;
   m->res.cap_halo = cap_halo;
   m->res.ctas = G;
   return TF_OK;
 }
 
-// Device bytes tf_resident_build may take, for budgeting.
+}  // namespace
+
+// Before a Jacobi / none solve: the first one of a matrix lays it out (a matrix
+// registered for other uses carries nothing of it).
+int tf_resident_prepare(tf_matrix_s* m) {
+  if (m->res.rows == 0 || m->res.ctas > 0) return TF_OK;
+  const int st = res_build(m);
+  if (m->res.ctas == 0) m->res.rows = 0;   // does not fit
+  return st;
+}
+
+// Device bytes tf_resident_prepare may take, for budgeting.
 size_t tf_resident_bytes(int n, int64_t nnz) {
   if (n < 1 || (size_t)nnz * 10 > (size_t)148 * kResSmemMax) return 0;
   return (size_t)nnz * 2 + (size_t)n * 28 + ((size_t)1 << 16);
@@ -619,13 +640,12 @@ int tf_resident_run(tf_matrix_s* m, int prec, const SolveParams* p, double* x, d
   return TF_OK;
 }
 
-// After a solve that gave up: the words of unfinished exchanges and the
-// recorded status.  Waited for: the matrix's next solve may run on another
-// context's stream (tf_pool.cu).
+// After a solve that gave up: the words of unfinished exchanges, and the recorded
+// status, which a resident solve polls but does not clear.  Waited for: the
+// matrix's next solve may run on another context's stream (tf_pool.cu).
 int tf_resident_reset(tf_matrix_s* m) {
-  if (!m->res.ctas) return TF_OK;
   cudaStream_t s = m->ctx->stream;
-  TF_CUDA_TRY(cudaMemsetAsync(m->res.words, 0, m->res.words_bytes, s));
+  if (m->res.ctas) TF_CUDA_TRY(cudaMemsetAsync(m->res.words, 0, m->res.words_bytes, s));
   TF_CUDA_TRY(cudaMemsetAsync(&m->d_state->status, 0, sizeof(int), s));
   for (auto* c : m->slices)
     if (c) TF_CUDA_TRY(cudaMemsetAsync(&c->d_state->status, 0, sizeof(int), s));

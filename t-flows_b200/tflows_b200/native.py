@@ -32,7 +32,8 @@ EXPORTS = [
     "tf_ctx_set_wait_limit", "tf_ctx_fail_allocs",
     "tf_host_pin", "tf_host_unpin", "tf_spmv", "tf_residual", "tf_nrms",
     "tf_ctx_sync", "tf_ctx_stream", "tf_last_error_message", "tf_matrix_tile_config",
-    "tf_matrix_row_patterns", "tf_matrix_renumbered", "tf_matrix_tuning",
+    "tf_matrix_row_patterns", "tf_matrix_renumbered", "tf_matrix_resident",
+    "tf_matrix_tuning",
     "tf_tuning_cache_clear", "tf_pool_cancel", "tf_server_cancel", "tf_matrix_icc_levels",
     "tf_vec_axpby", "tf_vec_gather", "tf_vec_scatter", "tf_vec_recip", "tf_vec_dot",
     "tf_vec_nrms_sum", "tf_vec_jacobi", "tf_vec_minmax",
@@ -102,6 +103,7 @@ def load(path=LIB_PATH):
     L.tf_vec_minmax.argtypes = [_vp, ci, _vp, _vp]
     L.tf_matrix_row_patterns.argtypes = [_vp]
     L.tf_matrix_renumbered.argtypes = [_vp]
+    L.tf_matrix_resident.argtypes = [_vp]
     solve_args = [_vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, ctypes.c_int,
                   _c_int_p, ctypes.c_double, _c_dbl_p, _c_dbl_p]
     L.tf_solve.argtypes = solve_args
@@ -288,6 +290,12 @@ class Matrix:
     def renumbered(self):
         """True when Jacobi / none solves run on a renumbered copy."""
         return bool(load().tf_matrix_renumbered(self.h))
+
+    @property
+    def resident_ctas(self):
+        """CTAs of the one-kernel Jacobi / none solve (0: not laid out yet, or
+        the solve is a graph of kernels)."""
+        return load().tf_matrix_resident(self.h)
 
     @property
     def row_patterns(self):

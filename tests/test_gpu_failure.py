@@ -61,6 +61,29 @@ def test_wait_limit_runs_out_then_context_recovers(kind, monkeypatch):
         ctx.close()
 
 
+def test_icc_solve_that_times_out_leaves_the_next_solves_alone():
+    """An ICC solve under a nanosecond's limit, before the matrix's first
+    one-kernel solve and after it: both kinds then solve normally."""
+    s = systems.small_hex(20, seed=4, kind="pressure", ratio=1.02)
+    ctx = native.Context(0)
+    m = native.Matrix(ctx, s.csr.row, s.csr.col, s.csr.dia)
+    try:
+        for _ in range(2):
+            ctx.set_wait_limit(1e-9)
+            with pytest.raises(native.TFError) as e:
+                gpu(ctx, m, s, s.val, s.b, 200, 1e-10, 1.0, "icc")
+            assert e.value.status == 4
+            ctx.set_wait_limit(0.0)
+            for prec in ("jacobi", "icc"):
+                x, it, res = gpu(ctx, m, s, s.val, s.b, 5000, 1e-10, 1.0, prec)
+                ox, oit, _ = oracle(s, s.val, s.b, 5000, 1e-10, 1.0, prec)
+                assert abs(it - oit) <= max(1, 0.02 * oit) and res < 1e-10
+                assert np.linalg.norm(x - ox) <= 1e-8 * np.linalg.norm(ox)
+    finally:
+        m.close()
+        ctx.close()
+
+
 def wide_halo_system(n=30000):
     """Symmetric and diagonally dominant; 256 consecutive rows refer to some 2,300
     rows outside them, more than the four a thread polls for ahead."""
