@@ -584,11 +584,16 @@ int res_build(tf_matrix_s* m) {
 }  // namespace
 
 // Before a Jacobi / none solve: the first one of a matrix lays it out (a matrix
-// registered for other uses carries nothing of it).
+// registered for other uses carries nothing of it).  Without room for that the
+// graph of kernels, which has its memory, solves the matrix.
 int tf_resident_prepare(tf_matrix_s* m) {
   if (m->res.rows == 0 || m->res.ctas > 0) return TF_OK;
-  const int st = res_build(m);
+  int st = res_build(m);
   if (m->res.ctas == 0) m->res.rows = 0;   // does not fit
+  if (st == TF_ERR_OOM) {
+    cudaGetLastError();   // not to be found by the next launch
+    st = TF_OK;
+  }
   return st;
 }
 

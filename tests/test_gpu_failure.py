@@ -183,6 +183,30 @@ def test_right_hand_sides_after_one_that_timed_out_are_left_alone():
         ctx.close()
 
 
+def test_solve_without_room_for_the_one_kernel_layout():
+    """The layout is an accelerator: where its memory is not to be had, the
+    graph of kernels solves the matrix, single and several right-hand sides."""
+    s = systems.small_hex(17, seed=3, kind="pressure", ratio=1.02)
+    want = oracle(s, s.val, s.b, 3000, 1e-10, 1.0)
+    with native.Context(0) as ctx:
+        for multi in (False, True):
+            m = native.Matrix(ctx, s.csr.row, s.csr.col, s.csr.dia)
+            try:
+                ctx.fail_allocs(0, 1)
+                if multi:
+                    X = np.stack([s.x0, s.x0])
+                    it, res = native.solve_multi(ctx, m, "cg", "jacobi", s.val.copy(), X,
+                                                 np.stack([s.b, s.b]), 3000, 1e-10, 1.0)
+                    x, it, res = X[1], it[1], res[1]
+                else:
+                    x, it, res = gpu(ctx, m, s, s.val, s.b, 3000, 1e-10, 1.0)
+                assert m.resident_ctas == 0
+                assert abs(it - want[1]) <= max(1, 0.02 * want[1]) and res < 1e-10
+                assert np.linalg.norm(x - want[0]) <= 1e-8 * np.linalg.norm(want[0])
+            finally:
+                m.close()
+
+
 def test_wait_limit_argument_checks(gpu_ctx):
     with pytest.raises(native.TFError):
         gpu_ctx.set_wait_limit(-1.0)
