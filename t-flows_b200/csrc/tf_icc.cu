@@ -125,7 +125,6 @@ void choose_layout(tf_matrix_s* m, int widest) {
 // The records of both sweeps, made on the device before the first ICC solve
 // of a matrix (a matrix that is never solved with ICC carries none).
 int pack(tf_matrix_s* m) {
-  if (m->icc_packed) return TF_OK;
   cudaStream_t s = m->ctx->stream;
   const std::vector<int>* ptrs[2] = {&m->h_levf_ptr, &m->h_levb_ptr};
   const int* rows[2] = {m->d_levf_rows, m->d_levb_rows};
@@ -213,7 +212,6 @@ int pack(tf_matrix_s* m) {
   const int st = build();
   for (int* q : {d_info, d_ptr[0], d_ptr[1], d_first[0], d_first[1], d_pos[0], d_pos[1]})
     tf_dev_free(m->ctx, q);
-  if (st == TF_OK) m->icc_packed = 1;
   return st;
 }
 
@@ -282,7 +280,7 @@ void plan_levels(tf_matrix_s* m, tf_icc_plan* p) {
 // Where k_residual and k_update store r for the one-CTA sweeps.
 IccResid tf_icc_resid(const tf_matrix_s* m) {
   IccResid r{};
-  if (m->icc_packed) {
+  if (m->icc_packed > 0) {
     r.idx_f = m->icc_dir[0].idx;
     r.idx_b = m->icc_dir[1].idx;
     r.rec_f = reinterpret_cast<double*>(m->icc_dir[0].rec);
@@ -295,16 +293,30 @@ size_t tf_icc_bytes(int n, int64_t nnz) {
   return (size_t)nnz * 18 + (size_t)n * 72 + ((size_t)1 << 16);
 }
 
-int tf_icc_prepare(tf_matrix_s* m) { return narrow_levels(m) ? pack(m) : TF_OK; }
+// Without room for the records (or with more entries than their 32-bit indices
+// name) the matrix keeps one kernel per level, which needs none.
+int tf_icc_prepare(tf_matrix_s* m) {
+  if (m->icc_packed != 0 || !narrow_levels(m)) return TF_OK;
+  int st = pack(m);
+  m->icc_packed = st == TF_OK ? 1 : -1;
+  if (st == TF_ERR_OOM) {
+    tf_icc_free(m);
+    cudaGetLastError();   // not to be found by the next launch
+    st = TF_OK;
+  }
+  return st;
+}
 
 void tf_icc_free(tf_matrix_s* m) {
-  for (auto& g : m->icc_dir)
+  for (auto& g : m->icc_dir) {
     for (void* q : {(void*)g.slice, (void*)g.chunk, (void*)g.src, (void*)g.idx, (void*)g.rec})
       tf_dev_free(m->ctx, q);
+    g = tf_icc_dir_s();
+  }
 }
 
 int tf_icc_make_plan(tf_matrix_s* m, tf_icc_plan* p) {
-  if (!m->icc_packed) {
+  if (m->icc_packed <= 0) {
     plan_levels(m, p);
     return TF_OK;
   }

@@ -168,7 +168,7 @@ struct tf_matrix_s {
   // The one-CTA sweeps' packed slices (tf_icc_prepare), made before the
   // first ICC solve of a matrix with narrow levels.
   tf_icc_dir_s icc_dir[2];       // forward, backward
-  int icc_packed = 0;
+  int icc_packed = 0;            // 1: made; -1: no room, one kernel per level
   int icc_width = 0, icc_batch = 0, icc_warps = 0, icc_stages = 0, icc_ring = 0;
   // cached graphs, one per (preconditioner, x update deferred or not)
   cudaGraphExec_t graph[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};

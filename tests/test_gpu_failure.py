@@ -207,6 +207,25 @@ def test_solve_without_room_for_the_one_kernel_layout():
                 m.close()
 
 
+@pytest.mark.parametrize("skip", [0, 1, 9, 13, 16])
+def test_icc_without_room_for_the_records(skip):
+    """Any allocation of the one-CTA sweeps' records that fails leaves the
+    kernels per level, which give every z the same bits; the sums over z are
+    taken in another order."""
+    s = systems.small_hex(14, seed=3, kind="pressure", ratio=1.02)
+    want = oracle(s, s.val, s.b, 3000, 1e-10, 1.0, "icc")
+    with native.Context(0) as ctx:
+        m = native.Matrix(ctx, s.csr.row, s.csr.col, s.csr.dia)
+        try:
+            ctx.fail_allocs(skip, 1)   # the records are 17 allocations
+            for _ in range(2):
+                x, it, res = gpu(ctx, m, s, s.val, s.b, 3000, 1e-10, 1.0, "icc")
+                assert it == want[1] and res < 1e-10
+                assert np.linalg.norm(x - want[0]) <= 1e-8 * np.linalg.norm(want[0])
+        finally:
+            m.close()
+
+
 def test_wait_limit_argument_checks(gpu_ctx):
     with pytest.raises(native.TFError):
         gpu_ctx.set_wait_limit(-1.0)
