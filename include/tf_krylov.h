@@ -199,8 +199,9 @@ int tf_last_history(tf_ctx ctx, double* hist, int cap, int* count);
  * much time since its start -- or once such a wait has been blocked that
  * long -- and the solve ends with TF_ERR_TIMEOUT.  The one-kernel solve of a
  * matrix that fits the chip stops when an exchange between its CTAs is not
- * complete this long after the one before it, and so do the waits of the ICC
- * sweeps.  Before a stopped CTA
+ * complete this long after the one before it; the ICC sweeps of one kernel
+ * stop when one of their waits has been blocked this long, however long the
+ * sweeps take.  Before a stopped CTA
  * exits it still waits for the copies it started (with the default limit),
  * and the context stays usable.  The reference has no counterpart (its
  * failures stop the run, Shared/Message_Mod/Error.f90:74). */

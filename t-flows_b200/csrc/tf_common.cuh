@@ -355,9 +355,8 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, unsigned parit
 }
 // A deadline whose looks mostly read the SM clock only: the global timer is read
 // at the first look after the limit starts to count and then only when
-// kLookCycles have passed since, so a limit is kept to within that (the one-CTA
-// ICC sweeps took 3 % longer with the timer read at every wait).  Once passed it
-// stays so until renewed: a wait that gave up early may leave it to the next
+// kLookCycles have passed since, so a limit is kept to within that.  Once passed
+// it stays so until renewed: a wait that gave up early may leave it to the next
 // look to end the kernel.
 struct Deadline {
   unsigned long long limit, ns;   // globaltimer
@@ -383,13 +382,6 @@ struct Deadline {
     look = 0;
   }
 };
-// mbar_wait_or_abort on such a deadline.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity,
-                                          volatile int* abort_flag, Deadline& deadline) {
-  while (!mbar_try_wait(bar, parity))
-    if (*abort_flag || deadline.passed()) return false;
-  return !deadline.passed();
-}
 // Wait for the bulk copies armed on `bar` before the CTA exits: always the
 // default limit (never the caller's), so a short caller limit cannot end a
 // CTA with copies into its shared memory still in flight.

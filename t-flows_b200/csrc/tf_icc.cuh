@@ -389,6 +389,29 @@ __device__ __forceinline__ int icc_progress(const int* progress) {
   return v;
 }
 
+
+struct IccPatience {
+  unsigned long long limit, until;
+  long long look;                    // SM clock at which to read the timer again
+  __device__ __forceinline__ explicit IccPatience(unsigned long long limit_ns)
+      : limit(limit_ns), until(0), look(0) {}
+  __device__ __forceinline__ bool over(bool first) {
+    const long long c = clock64();
+    if (!first && c < look) return false;
+    look = c + Deadline::kLookCycles;
+    if (first) until = deadline_after(limit);
+    return globaltimer_ns() > until;
+  }
+};
+// False at the limit, or once *abort_flag is set.
+__device__ __forceinline__ bool icc_wait(uint64_t* bar, unsigned parity, volatile int* abort_flag,
+                                         unsigned long long limit) {
+  IccPatience patience(limit);
+  for (bool first = true; !mbar_try_wait(bar, parity); first = false)
+    if (*abort_flag || patience.over(first)) return false;
+  return true;
+}
+
 // One sweep.  `it0` chunks have gone through the stages before it (returned
 // count: after it).  K entries of a row, in batches of B, are loaded ahead,
 // the rest of its packed width is read from the stage, and what is longer
@@ -396,7 +419,7 @@ __device__ __forceinline__ int icc_progress(const int* progress) {
 template <int KIND, int K, int B, int W>
 __device__ __forceinline__ int icc_sweep(const IccArgs& a, unsigned char* smem,
                                          const IccLayout& L, int it0, bool& ok,
-                                         Deadline& deadline, double& rho) {
+                                         unsigned long long limit, double& rho) {
   static_assert(W % kIccChunk == 0, "a warp's slices lie whole chunks apart");
   const IccDir& g = KIND == kIccBackward ? a.b : a.f;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -423,7 +446,7 @@ __device__ __forceinline__ int icc_sweep(const IccArgs& a, unsigned char* smem,
       for (int m = m0; m < nchunks; m += step) {
         const int2 nxt2 = m + 2 * step < nchunks ? __ldg(g.chunk + m + 2 * step) : c;
         if (it0 + m >= stages) {
-          if (!mbar_wait(&empty[stage], par, abort_flag, deadline)) {
+          if (!icc_wait(&empty[stage], par, abort_flag, limit)) {
             ok = false;
             *abort_flag = 1;
             break;
@@ -468,7 +491,7 @@ __device__ __forceinline__ int icc_sweep(const IccArgs& a, unsigned char* smem,
     for (int s = warp; s < g.nslices; s += W) {
       // What does not depend on other rows.
       bool here = mbar_try_wait(&full[stage], par) ||
-                  mbar_wait(&full[stage], par, abort_flag, deadline);
+                  icc_wait(&full[stage], par, abort_flag, limit);
       if (!__all_sync(0xffffffffu, here)) {
         ok = false;
         *abort_flag = 1;
@@ -499,8 +522,9 @@ __device__ __forceinline__ int icc_sweep(const IccArgs& a, unsigned char* smem,
           }
       }
       // The earlier levels.
+      IccPatience patience(limit);
       for (int spin = 0; icc_progress(progress) < m.first; ++spin)
-        if ((spin & 63) == 63 && (*abort_flag || deadline.passed())) {
+        if ((spin & 63) == 63 && (*abort_flag || patience.over(spin == 63))) {
           here = false;
           break;
         }
@@ -596,8 +620,8 @@ static __global__ void __launch_bounds__(32 * (W + kIccProducers), 1) k_icc_form
   icc_init(a, tf_icc_smem, L);
   bool ok = true;
   double none = 0.0;
-  Deadline deadline(wait_limit(a.prm));
-  icc_sweep<kIccForm, K, B, W>(a, tf_icc_smem, L, 0, ok, deadline, none);
+  const unsigned long long limit = wait_limit(a.prm);
+  icc_sweep<kIccForm, K, B, W>(a, tf_icc_smem, L, 0, ok, limit, none);
   if (!ok) atomicExch(&a.st->status, (int)TF_ERR_TIMEOUT);
 }
 
@@ -612,17 +636,17 @@ static __global__ void __launch_bounds__(32 * (W + kIccProducers), 1) k_icc_appl
   if (st->done) return;
   const IccLayout L(a.width, a.stages, a.ring);
   icc_init(a, tf_icc_smem, L);
-  Deadline deadline(wait_limit(a.prm));
+  const unsigned long long limit = wait_limit(a.prm);
   bool ok = true;
   double rho = 0.0;
-  int it = icc_sweep<kIccForward, K, B, W>(a, tf_icc_smem, L, 0, ok, deadline, rho);
+  int it = icc_sweep<kIccForward, K, B, W>(a, tf_icc_smem, L, 0, ok, limit, rho);
   // the backward sweep's bulk copies read what these threads have stored
   asm volatile("fence.proxy.async;" ::: "memory");
   ok = !__syncthreads_or(!ok);
   if (threadIdx.x == 0)
     *reinterpret_cast<int*>(tf_icc_smem + L.bar_at + 16 * a.stages) = 0;   // progress
   __syncthreads();
-  if (ok) icc_sweep<kIccBackward, K, B, W>(a, tf_icc_smem, L, it, ok, deadline, rho);
+  if (ok) icc_sweep<kIccBackward, K, B, W>(a, tf_icc_smem, L, it, ok, limit, rho);
   if (!ok) atomicExch(&st->status, (int)TF_ERR_TIMEOUT);
   rho = block_red<kSum>(rho, scratch);
   if (threadIdx.x == 0) {

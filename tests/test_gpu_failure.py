@@ -84,6 +84,33 @@ def test_icc_solve_that_times_out_leaves_the_next_solves_alone():
         ctx.close()
 
 
+def test_icc_sweeps_longer_than_the_limit_run_to_their_end():
+    """100,000 levels of one row take some 30 ms a sweep, the products a few us:
+    a limit of 5 ms is about waits that nothing moves, not about long sweeps."""
+    n = 100000
+    i = np.arange(n)
+    lo, up = i > 0, i < n - 1
+    w = -np.random.default_rng(5).uniform(0.2, 1.0, n)   # entry (i, i + 1)
+    diag = 0.3 - w * up - np.roll(w, 1) * lo
+    col = np.stack([i, i - 1, i + 1], 1)
+    val = np.stack([diag, np.roll(w, 1), w], 1)
+    keep = np.stack([i >= 0, lo, up], 1)
+    row = np.concatenate([[1], 1 + np.cumsum(keep.sum(1))]).astype(np.int32)
+    col, val = (col[keep] + 1).astype(np.int32), val[keep]
+    b = np.random.default_rng(6).uniform(-1, 1, n)
+    ox, ov, ob = np.zeros(n), val.copy(), b.copy()
+    want = O.solve_native("cg", "icc", row, col, row[:-1].copy(), ov, ox, ob, 5, 1e-12, norm=1.0)
+    with native.Context(0) as ctx:
+        m = native.Matrix(ctx, row, col, row[:-1].copy())
+        try:
+            ctx.set_wait_limit(5e-3)
+            x, v, bb = np.zeros(n), val.copy(), b.copy()
+            it, res = native.solve(ctx, m, "cg", "icc", v, x, bb, 5, 1e-12, 1.0)
+        finally:
+            m.close()
+    assert it == want["niter"] and np.linalg.norm(x - ox) <= 1e-8 * np.linalg.norm(ox)
+
+
 def wide_halo_system(n=30000):
     """Symmetric and diagonally dominant; 256 consecutive rows refer to some 2,300
     rows outside them, more than the four a thread polls for ahead."""
