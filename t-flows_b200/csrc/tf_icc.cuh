@@ -389,7 +389,11 @@ __device__ __forceinline__ int icc_progress(const int* progress) {
   return v;
 }
 
-
+// A sweep's blocked waits: each may last `limit` ns (from its first look, to
+// within a few us), so a sweep of many levels takes as long as it takes.  The
+// limit counts within a wait, and nothing of it is held between waits (counting
+// from the last finished slice cost 1 to 4 % of an iteration, reading the timer
+// at every wait 3 %).
 struct IccPatience {
   unsigned long long limit, until;
   long long look;                    // SM clock at which to read the timer again
