@@ -111,6 +111,11 @@ int tf_tuning_cache_clear(void);
  * Prec_Solve.f90:67-92's recurrences): forward and backward counts, 0 when
  * ICC is unavailable (diagonal not first).  No reference counterpart. */
 int tf_matrix_icc_levels(tf_matrix m, int* forward, int* backward);
+/* Kernels that apply the incomplete-Cholesky preconditioner once: 1 (one CTA
+ * walks all levels; few rows and entries a level) or one per level and one for
+ * rho; 0 when ICC is unavailable.  TF_ICC_SWEEPS=one or =levels in the
+ * environment of the registration asks for either.  No reference counterpart. */
+int tf_matrix_icc_kernels(tf_matrix m);
 /* Number of row patterns of the compressed column layout chosen at
  * registration (rows whose column offsets relative to the row index repeat,
  * as on structured hex blocks: one byte per row instead of four per entry;

@@ -613,6 +613,12 @@ extern "C" int tf_matrix_icc_levels(tf_matrix m, int* forward, int* backward) {
   TF_API_END
 }
 
+extern "C" int tf_matrix_icc_kernels(tf_matrix m) {
+  TF_API_BEGIN
+  return m ? tf_icc_kernels(m) : TF_ERR_ARG;
+  TF_API_END
+}
+
 extern "C" int tf_tuning_cache_clear(void) {
   TF_API_BEGIN
   tf_tune_cache_clear();

@@ -32,29 +32,45 @@ void bucket(const std::vector<int>& lev, int nlev, std::vector<int>& ptr,
 // ...; if(k > i) exit`; backward: for the upper entries visited from the
 // row's end down to `if(k < i) exit`, owned rows only (k <= ni).
 int tf_icc_build(tf_matrix_s* m, const int* row0, const int* col0) {
+  if (const char* form = getenv("TF_ICC_SWEEPS"))   // "one" CTA, or a kernel per level
+    m->icc_form = form[0] == 'o' ? 1 : -1;
   const int ni = m->ni;
   std::vector<int> levf(ni, 0), levb(ni, 0);
   int nf = 0, nb = 0;
+  // Entries the sweeps visit, and levels with a row longer than is packed.
+  std::vector<char> longf(ni, 0), longb(ni, 0);
+  m->icc_entries = 0;
+  auto count = [&](std::vector<char>& lev, int l, int len) {
+    m->icc_entries += len;
+    if (len > kIccWidth) lev[l] = 1;
+  };
   for (int i = 0; i < ni; ++i) {
-    int l = 0;
+    int l = 0, len = 0;
     for (int j = row0[i] + 1; j < row0[i + 1]; ++j) {
       const int k = col0[j];
       if (k > i) break;
       l = std::max(l, levf[k] + 1);
+      ++len;
     }
     levf[i] = l;
     nf = std::max(nf, l + 1);
+    count(longf, l, len);
   }
   for (int i = ni - 1; i >= 0; --i) {
-    int l = 0;
+    int l = 0, len = 0;
     for (int j = row0[i + 1] - 1; j >= row0[i] + 1; --j) {
       const int k = col0[j];
       if (k < i) break;
-      if (k < ni) l = std::max(l, levb[k] + 1);
+      if (k >= ni) continue;
+      l = std::max(l, levb[k] + 1);
+      ++len;
     }
     levb[i] = l;
     nb = std::max(nb, l + 1);
+    count(longb, l, len);
   }
+  m->icc_long_levels = (int)(std::count(longf.begin(), longf.end(), 1) +
+                             std::count(longb.begin(), longb.end(), 1));
   std::vector<int> rf, rb;
   bucket(levf, nf, m->h_levf_ptr, rf);
   bucket(levb, nb, m->h_levb_ptr, rb);
@@ -103,11 +119,14 @@ int dev_array(tf_matrix_s* m, T** p, size_t count) {
   return st;
 }
 
-// Rows per level, on average over both sweeps, up to which one CTA walks the
-// levels.
+// Whether one CTA walks the levels: by rows and entries a level, on average over
+// both sweeps (kIccOneRows and what follows it).
 bool narrow_levels(const tf_matrix_s* m) {
+  if (m->icc_form != 0) return m->icc_form > 0;
   const long long levels = (long long)(m->h_levf_ptr.size() + m->h_levb_ptr.size()) - 2;
-  return 2LL * m->ni <= kIccOneRows * levels;
+  const bool long_rows = 8LL * m->icc_long_levels > levels;
+  return 2LL * m->ni <= kIccOneRows * levels &&
+         m->icc_entries <= (long_rows ? kIccOneLongEntries : kIccOneEntries) * levels;
 }
 
 // Batch, packed width, consumer warps, stages and ring slots for the widest
@@ -313,6 +332,12 @@ void tf_icc_free(tf_matrix_s* m) {
       tf_dev_free(m->ctx, q);
     g = tf_icc_dir_s();
   }
+}
+
+int tf_icc_kernels(const tf_matrix_s* m) {
+  if (!m->icc_ready) return 0;
+  const bool one = m->icc_packed > 0 || (m->icc_packed == 0 && narrow_levels(m));
+  return one ? 1 : (int)(m->h_levf_ptr.size() + m->h_levb_ptr.size()) - 2 + 1;
 }
 
 int tf_icc_make_plan(tf_matrix_s* m, tf_icc_plan* p) {

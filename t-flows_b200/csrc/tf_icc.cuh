@@ -327,13 +327,23 @@ static __global__ void __launch_bounds__(256) k_icc_pack(IccArgs a) {
 
 // Shared memory of the sweeping CTA at most.
 constexpr int kIccSmemBytes = 225 * 1024;
-// Mean rows per level up to which one CTA walks the levels.  One Cg iteration,
-// us, one kernel per level / one CTA: 57x43x53 hex (860 rows a level) 1259 /
-// 361, 64^3 (1380) 1592 / 647, 76^3 (1940) 2167 / 1655, polyhedral 21 k cells
-// (81) 3396 / 274, 100 k (232) 6239 / 884, 400 k (578) 13746 / 6262.  At 100^3
-// (3355 rows a level) two levels no longer fit the ring of results and one SM
-// takes 5272 against 4236.
-constexpr long long kIccOneRows = 2000;
+// Up to how many rows and entries a level, on average, one CTA walks the levels.
+// One CTA pays 0.3 to 1.3 us for 1,000 entries (the more neighbours lie far
+// back, the more), a kernel per level 5 to 14 us a level whatever it holds.  One
+// Cg iteration, us, a kernel per level / one CTA, at rows and entries a level:
+//   hex 57x43x53    860  2,500   1259 /  361   polyhedral 100 k  232  1,560   6239 /   884
+//   hex 64^3      1,380  4,070   1826 /  713   400 k             578  3,950  15275 /  6567
+//   hex 76^3      1,942  5,750   2481 / 1796   1.0 M           1,067  7,340  25489 / 17707
+//   hex 92^3      2,842  8,430   4089 / 3907   1.4 M           1,319  9,090  29612 / 23660
+//   hex 100^3     3,356  9,970   4664 / 5689   2.0 M           1,674 11,560  33927 / 34502
+constexpr long long kIccOneRows = 2000, kIccOneEntries = 11000;
+// ... and where more than an eighth of the levels hold a row with more entries
+// than are packed (kIccWidth): such a row is summed from global memory, about as
+// long as a kernel per level takes for its level, so everything else of the level
+// comes on top.  Levels of rows of 7 entries, one in a hundred of 22: 300 rows
+// (2,110 entries) 858 / 480, 800 (5,630) 880 / 967, 1,600 (11,250) 903 / 1724;
+// Delaunay duals (0.3 % of the rows) of 150,000 cells, 1,770 entries, 12673 / 5200.
+constexpr long long kIccOneLongEntries = 4000;
 
 // ---------------------------------------------------------------------------
 // All levels in one CTA

@@ -163,11 +163,14 @@ struct tf_matrix_s {
   int* d_levf_rows = nullptr;  // forward-sweep rows grouped by level
   int* d_levb_rows = nullptr;  // backward-sweep rows grouped by level
   std::vector<int> h_levf_ptr, h_levb_ptr;
+  long long icc_entries = 0;   // entries both sweeps visit
+  int icc_long_levels = 0;     // levels with a row of more than kIccWidth of them
   double* d_icc_d = nullptr;     // Prec_Form's d
   double* d_icc_dinv = nullptr;  // Prec_Form's d_inv
   // The one-CTA sweeps' packed slices (tf_icc_prepare), made before the
   // first ICC solve of a matrix with narrow levels.
   tf_icc_dir_s icc_dir[2];       // forward, backward
+  int icc_form = 0;    // asked for at registration (TF_ICC_SWEEPS): 1 one CTA, -1 levels
   int icc_packed = 0;            // 1: made; -1: no room, one kernel per level
   int icc_width = 0, icc_batch = 0, icc_warps = 0, icc_stages = 0, icc_ring = 0;
   // cached graphs, one per (preconditioner, x update deferred or not)
@@ -242,6 +245,7 @@ int tf_resident_reset(tf_matrix_s* m);
 bool tf_resident(const tf_matrix_s* m);
 int tf_icc_build(tf_matrix_s* m, const int* h_row0, const int* h_col0);
 int tf_icc_prepare(tf_matrix_s* m);   // before a solve with ICC
+int tf_icc_kernels(const tf_matrix_s* m);   // that apply the preconditioner once
 void tf_icc_free(tf_matrix_s* m);
 size_t tf_icc_bytes(int n, int64_t nnz);   // the records of both sweeps, for budgeting
 tf::IccResid tf_icc_resid(const tf_matrix_s* m);

@@ -35,6 +35,7 @@ EXPORTS = [
     "tf_matrix_row_patterns", "tf_matrix_renumbered", "tf_matrix_resident",
     "tf_matrix_tuning",
     "tf_tuning_cache_clear", "tf_pool_cancel", "tf_server_cancel", "tf_matrix_icc_levels",
+    "tf_matrix_icc_kernels",
     "tf_vec_axpby", "tf_vec_gather", "tf_vec_scatter", "tf_vec_recip", "tf_vec_dot",
     "tf_vec_nrms_sum", "tf_vec_jacobi", "tf_vec_minmax",
     "tf_faces_register", "tf_assemble_pressure", "tf_assemble_momentum",
@@ -92,6 +93,7 @@ def load(path=LIB_PATH):
     L.tf_matrix_tile_config.argtypes = [_vp]
     L.tf_matrix_tuning.argtypes = [_vp, _c_int_p, _c_dbl_p, ctypes.c_int, _c_int_p]
     L.tf_matrix_icc_levels.argtypes = [_vp, _c_int_p, _c_int_p]
+    L.tf_matrix_icc_kernels.argtypes = [_vp]
     ci, cd = ctypes.c_int, ctypes.c_double
     L.tf_vec_axpby.argtypes = [_vp, ci, cd, _vp, cd, _vp, ci]
     L.tf_vec_gather.argtypes = [_vp, ci, _vp, _vp, _vp]
@@ -278,13 +280,16 @@ class Matrix:
                "tf_matrix_icc_levels")
         return f.value, b.value
 
+    @property
+    def icc_kernels(self):
+        """Kernels that apply the incomplete-Cholesky preconditioner once: 1, or
+        one per level and the rho reduction."""
+        return load().tf_matrix_icc_kernels(self.h)
+
     def icc_launches_per_iteration(self):
         """Kernel launches of one ICC-preconditioned Cg iteration: the three
-        iteration kernels and the sweeps -- one kernel when the levels have at
-        most 2,000 rows on average, else one per level and the rho
-        reduction."""
-        f, b = self.icc_levels()
-        return 4 if 2 * self.n_own <= 2000 * (f + b) else 3 + f + b + 1
+        iteration kernels and the preconditioner's."""
+        return 3 + self.icc_kernels
 
     @property
     def renumbered(self):

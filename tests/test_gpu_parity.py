@@ -582,25 +582,6 @@ def test_icc_parity_medium_and_poly(gpu_ctx):
     check_parity(gpu_solve(gpu_ctx, *args), oracle_solve(*args), 1e-10)
 
 
-@pytest.mark.parametrize("kind", ["hex", "poly"])
-def test_icc_persistent_sweeps_equal_level_kernels(gpu_ctx, kind, monkeypatch):
-    """The persistent ICC sweeps (one cooperative kernel per sweep, a grid
-    barrier between levels; opt-in) give the per-level kernels' bits."""
-    if kind == "hex":
-        s = systems.small_hex(30, seed=4, kind="pressure", ratio=1.03)
-    else:
-        s = systems.poly_system(20000, seed=6, kind="pressure", tol=1e-10, miter=3000,
-                                norm=1.0)
-    args = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b, s.x0, "cg", "icc", 3000, 1e-10, 1.0)
-    g1 = gpu_solve(gpu_ctx, *args)
-    monkeypatch.setenv("TF_ICC_PERSISTENT", "1")
-    g2 = gpu_solve(gpu_ctx, *args)
-    assert g1[3] == g2[3] and g1[4] == g2[4]
-    for u, w in zip(g1[:3], g2[:3]):
-        assert np.array_equal(u, w)
-    check_parity(g1, oracle_solve(*args), 1e-10)
-
-
 def test_icc_needs_diagonal_first(gpu_ctx):
     """The 4x4 example of Matrix_Mod.f90 stores rows in column order."""
     from golden.make_golden import example_4x4
@@ -633,26 +614,111 @@ def _band_system(n, offsets, seed):
     return row, np.array(col, np.int32), row[:-1].copy(), np.array(val), rng.uniform(-1, 1, n)
 
 
-@pytest.mark.parametrize("case", ["one-row", "slices", "hex-4-warps", "long-rows", "far",
-                                  "wide-levels"])
+def _layer_system(rows, layers, entries, long_share=0.0, seed=3):
+    """`layers` levels of `rows` rows, each row coupled to `entries` rows of the
+    layer before it (22 for a share of the rows): symmetric, diagonal first."""
+    rng = np.random.default_rng(seed)
+    n = rows * layers
+    width = np.where(rng.random(n) < long_share, 22, entries)
+    width[:rows] = 0
+    r = np.repeat(np.arange(n), width)
+    o = np.arange(len(r)) - np.repeat(np.cumsum(width) - width, width)
+    c = (r // rows - 1) * rows + (r % rows + o) % rows
+    v = -rng.uniform(0.2, 1.0, len(r))
+    diag = 0.3 - np.bincount(r, v, n) - np.bincount(c, v, n)
+    i = np.arange(n)
+    r, c, v = (np.concatenate(t) for t in ((r, c, i), (c, r, i), (v, v, diag)))
+    order = np.lexsort((c, c != r, r))
+    row = np.concatenate([[1], 1 + np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+    return (row, (c[order] + 1).astype(np.int32), row[:-1].copy(), v[order],
+            rng.uniform(-1, 1, n))
+
+
+def _icc_case(case):
+    if case in ("two-rows", "slices", "hex-3-lower"):
+        from tflows_b200.grids import hex_grid
+        dims = {"two-rows": (1, 1, 2), "slices": (33, 32, 3), "hex-3-lower": (17, 13, 11)}[case]
+        s = systems.pressure_system(hex_grid(*dims), 3, tol=1e-10, miter=500)
+        return s.csr.row, s.csr.col, s.csr.dia, s.val, s.b
+    if case == "poly":
+        s = systems.poly_system(20000, seed=6, kind="pressure", tol=1e-10, miter=3000, norm=1.0)
+        return s.csr.row, s.csr.col, s.csr.dia, s.val, s.b
+    if case == "wide-levels":   # two levels of 2,100 rows
+        return _band_system(4200, [2100], 7)
+    n, offsets, seed = {"one-row": (1, [], 4), "4-lower": (5000, [1, 5, 70, 900], 5),
+                        "12-lower": (4000, list(range(3, 15)), 5),
+                        "long-rows": (900, list(range(1, 41)), 5),
+                        "far": (12000, [4, 9000], 6)}[case]
+    return _band_system(n, offsets, seed)
+
+
+ICC_CASES = ["one-row", "two-rows", "slices", "hex-3-lower", "4-lower", "12-lower", "long-rows",
+             "far", "poly"]
+
+
+@pytest.mark.parametrize("case", ICC_CASES + ["wide-levels"])
 def test_icc_sweeps_at_their_edges(gpu_ctx, case):
     """The one-CTA sweeps where they can go wrong -- one row, levels of 31 to
-    33 rows, rows longer than the packed width (40 entries a side), results
-    older than the ring (9,000 positions back) -- and the kernel per level of
-    wide levels.  Row sums are the reference's, so the iterations are equal."""
-    if case in ("one-row", "slices", "hex-4-warps"):
-        from tflows_b200.grids import hex_grid
-        dims = {"one-row": (1, 1, 2), "slices": (33, 32, 3), "hex-4-warps": (17, 13, 11)}[case]
-        s = systems.pressure_system(hex_grid(*dims), 3, tol=1e-10, miter=500)
-        a = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b)
-    elif case == "long-rows":
-        a = _band_system(900, list(range(1, 41)), 5)
-    elif case == "far":
-        a = _band_system(12000, [4, 9000], 6)
-    else:   # two levels of 2,100 rows
-        a = _band_system(4200, [2100], 7)
+    33 rows, rows of each packed width and longer ones (40 entries a side),
+    results older than the ring (9,000 positions back) -- and the kernel per
+    level of wide levels.  Row sums are the reference's, so the iterations are
+    equal."""
+    a = _icc_case(case)
     n = len(a[4])
+    m = native.Matrix(gpu_ctx, *a[:3])
+    try:
+        assert m.icc_kernels == (1 if case != "wide-levels" else sum(m.icc_levels()) + 1)
+    finally:
+        m.close()
     args = (*a, np.zeros(n), "cg", "icc", 300, 1e-10, 1.0)
+    check_parity(gpu_solve(gpu_ctx, *args), oracle_solve(*args), 1e-10,
+                 exact_iters=case != "poly")
+
+
+@pytest.mark.parametrize("case", ICC_CASES)
+def test_icc_sweep_forms_give_the_same_bits(gpu_ctx, case, monkeypatch):
+    """z of the one-CTA sweeps and of the kernels per level is the same bit for
+    bit; rho, its product with r, is summed in another order.  After one
+    iteration from x = 0 x is alfa z: for right-hand sides whose alfa comes out
+    equal x is, too, and alfa differs in its last bits otherwise."""
+    a = _icc_case(case)
+    n = len(a[4])
+    rng = np.random.default_rng(12)
+    got = {}
+    B = [rng.uniform(-1, 1, n) for _ in range(24)]
+    for form in ("one", "levels"):
+        monkeypatch.setenv("TF_ICC_SWEEPS", form)
+        m = native.Matrix(gpu_ctx, *a[:3])
+        try:
+            assert (m.icc_kernels == 1) == (form == "one")
+            got[form] = []
+            for b in B:
+                v, x, bb = a[3].copy(), np.zeros(n), b.copy()
+                it, _ = native.solve(gpu_ctx, m, "cg", "icc", v, x, bb, 1, 1e-300, 1.0)
+                assert it == 1
+                got[form].append(x)
+        finally:
+            m.close()
+    same = [np.array_equal(x, y) for x, y in zip(got["one"], got["levels"])]
+    assert any(same)
+    for x, y in zip(got["one"], got["levels"]):
+        assert np.allclose(x, y, rtol=1e-13, atol=0)
+
+
+@pytest.mark.parametrize("rows,layers,entries,long_share,one", [
+    (300, 12, 7, 0.0, True), (300, 12, 7, 0.05, True), (800, 6, 7, 0.0, True),
+    (800, 6, 7, 0.05, False), (1900, 6, 4, 0.0, True), (1900, 6, 8, 0.0, False),
+    (2100, 6, 1, 0.0, False)])
+def test_icc_form_follows_rows_entries_and_long_rows(gpu_ctx, rows, layers, entries, long_share,
+                                                     one):
+    a = _layer_system(rows, layers, entries, long_share)
+    m = native.Matrix(gpu_ctx, *a[:3])
+    try:
+        f, b = m.icc_levels()
+        assert f == layers and m.icc_kernels == (1 if one else f + b + 1)
+    finally:
+        m.close()
+    args = (*a, np.zeros(len(a[4])), "cg", "icc", 300, 1e-10, 1.0)
     check_parity(gpu_solve(gpu_ctx, *args), oracle_solve(*args), 1e-10, exact_iters=True)
 
 
