@@ -9,7 +9,7 @@ from tflows_b200 import native
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2, 7, 2047, 2048, 2049, 300001])
+@pytest.mark.parametrize("n", [1, 2, 7, 2047, 2048, 2049, 300001, 1300001])
 def test_vec_kernels(gpu_ctx, n):
     import torch
     rng = np.random.default_rng(n)
