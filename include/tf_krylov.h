@@ -383,7 +383,9 @@ int tf_server_destroy(tf_server s);
  *  and released, so independent solves overlap on the GPU.  Requests are
  *  admitted in arrival order while the device bytes in flight stay within
  *  mem_budget (0: 20 GiB); one larger than the budget fails with
- *  TF_ERR_OOM.  Submit returns at once; wait blocks
+ *  TF_ERR_OOM.  One that fits without the memory of the one-kernel solve (or
+ *  the ICC sweeps of one kernel) but not with it is solved without: its sums
+ *  are then taken in another order than tf_solve's.  Submit returns at once; wait blocks
  *  until the request finished and reports end-to-end and queueing latency
  *  in milliseconds.  All pool functions are thread-safe.
  * ------------------------------------------------------------------------- */

@@ -109,13 +109,15 @@ void cut_slices(const std::vector<int>& ptr, std::vector<int4>& meta, std::vecto
   }
 }
 
+// An array of the records, within what the matrix may hold beside its own.
 template <class T>
 int dev_array(tf_matrix_s* m, T** p, size_t count) {
-  tf_dev_free(m->ctx, *p);   // an earlier attempt's
-  *p = nullptr;
+  const size_t bytes = (count + 8) * sizeof(T);
+  if (m->extra_bytes + m->icc_bytes + bytes > m->extra_limit) return TF_ERR_OOM;
   void* v = nullptr;
-  const int st = tf_dev_alloc_bytes(m->ctx, &v, (count + 8) * sizeof(T));
+  const int st = tf_dev_alloc_bytes(m->ctx, &v, bytes);
   *p = static_cast<T*>(v);
+  if (st == TF_OK) m->icc_bytes += bytes;
   return st;
 }
 
@@ -228,6 +230,7 @@ int pack(tf_matrix_s* m) {
     for (int k = 0; k < 2; ++k) m->icc_dir[k].far_any = info.far_any[k];
     return TF_OK;
   };
+  tf_icc_free(m);   // an earlier attempt's
   const int st = build();
   for (int* q : {d_info, d_ptr[0], d_ptr[1], d_first[0], d_first[1], d_pos[0], d_pos[1]})
     tf_dev_free(m->ctx, q);
@@ -308,8 +311,10 @@ IccResid tf_icc_resid(const tf_matrix_s* m) {
   return r;
 }
 
+// Entries padded to twice their number, and all that a row takes in both
+// directions where every level, and so every slice, is one row.
 size_t tf_icc_bytes(int n, int64_t nnz) {
-  return (size_t)nnz * 18 + (size_t)n * 72 + ((size_t)1 << 16);
+  return (size_t)nnz * 32 + (size_t)n * 256 + ((size_t)1 << 16);
 }
 
 // Without room for the records (or with more entries than their 32-bit indices
@@ -332,6 +337,7 @@ void tf_icc_free(tf_matrix_s* m) {
       tf_dev_free(m->ctx, q);
     g = tf_icc_dir_s();
   }
+  m->icc_bytes = 0;
 }
 
 int tf_icc_kernels(const tf_matrix_s* m) {

@@ -185,6 +185,9 @@ struct tf_matrix_s {
   int async_alloc = 0;   // device arrays from cudaMallocAsync on ctx->stream
   int host_lent = 0;     // h_state / h_params belong to the context
   size_t dev_bytes = 0;  // device bytes this matrix holds (with `ren`)
+  // What the one-kernel solve's layout holds besides, and the ICC records (their
+  // making's temporaries included); neither is made beyond extra_limit.
+  size_t extra_bytes = 0, icc_bytes = 0, extra_limit = SIZE_MAX;
   // Renumbered copy for the Jacobi / none solves (tf_renumber.cu): row i'
   // of `ren` is row perm[i'] here, entry j' of `ren` is entry src[j'].
   tf_matrix_s* ren = nullptr;
@@ -237,7 +240,7 @@ int tf_fp64_nrms(tf_matrix_s* m, const double* val, const double* r,
                  const double* x, int has_norm, double norm, double* out);
 void tf_resident_plan(tf_matrix_s* m, const int* row0);   // at registration
 int tf_resident_prepare(tf_matrix_s* m);   // before a solve without ICC
-size_t tf_resident_bytes(int n, int64_t nnz);
+size_t tf_resident_bytes(int n, int64_t nnz, const int* row, bool renumbered, int sms);
 int tf_resident_run(tf_matrix_s* m, int prec, const tf::SolveParams* p, double* x, double* b,
                     tf::SolveState* st, const tf::SolveState* before, int write_val);
 int tf_resident_reset(tf_matrix_s* m);
@@ -247,7 +250,7 @@ int tf_icc_build(tf_matrix_s* m, const int* h_row0, const int* h_col0);
 int tf_icc_prepare(tf_matrix_s* m);   // before a solve with ICC
 int tf_icc_kernels(const tf_matrix_s* m);   // that apply the preconditioner once
 void tf_icc_free(tf_matrix_s* m);
-size_t tf_icc_bytes(int n, int64_t nnz);   // the records of both sweeps, for budgeting
+size_t tf_icc_bytes(int n, int64_t nnz);   // what the sweeps' records may take, for budgeting
 tf::IccResid tf_icc_resid(const tf_matrix_s* m);
 // Registration behind tf_matrix_register; want_icc = 0 skips the ICC level
 // schedule.  Device bytes the matrix will hold, for budgeting.

@@ -65,7 +65,7 @@ struct PoolReq {
   double tol = 0.0;
   int has_norm = 0;
   double norm = 0.0;
-  size_t bytes = 0;
+  size_t bytes = 0, extra = 0;   // budgeted; of it for layouts that make solves faster
   uint64_t key = 0;           // structure key (pointers, sizes, sampled contents)
   Clock::time_point t_submit, t_start, t_done;
   int status = TF_OK;
@@ -183,6 +183,8 @@ struct tf_pool_s {
                             &m);
       if (st != TF_OK) return st;
       *pm = m;
+      m->extra_limit = r.extra;
+      if (m->ren) m->ren->extra_limit = r.extra;
     }
     cudaStream_t s = ctx->stream;
     const size_t vb = (size_t)r.nnz * 8, nb = (size_t)r.n * 8;
@@ -249,7 +251,11 @@ struct tf_pool_s {
           Held e;
           e.key = r->key;
           e.m = m;
-          e.bytes = r->bytes;
+          // what the layouts turned out to take
+          const size_t extra = m->extra_bytes + m->icc_bytes + (m->ren ? m->ren->extra_bytes : 0);
+          m->extra_limit = m->extra_bytes + m->icc_bytes;
+          e.bytes = r->bytes - r->extra + extra;
+          used -= r->extra - extra;
           e.last = ++tick;
           held.push_back(e);
         } else {
@@ -327,7 +333,12 @@ extern "C" int tf_pool_submit(tf_pool p, int solver, int prec, int n, int64_t nn
   r->tol = tol;
   r->has_norm = norm ? 1 : 0;
   r->norm = norm ? *norm : 0.0;
-  r->bytes = tf_matrix_bytes_for(n, nnz, row, col) +
+  const size_t plain = tf_matrix_bytes(n, nnz), made = tf_matrix_bytes_for(n, nnz, row, col);
+  const size_t extra =
+      prec == TF_PREC_ICC
+          ? tf_icc_bytes(n, nnz)
+          : tf_resident_bytes(n, nnz, row, made > plain, p->ctxs[0]->sm_count);
+  r->bytes = made +
              (prec == TF_PREC_ICC ? (size_t)n * 40 + 4096 : 0);
   r->key = structure_key(n, nnz, row, col, dia, prec == TF_PREC_ICC);
   std::lock_guard<std::mutex> lk(p->mu);
@@ -336,11 +347,13 @@ extern "C" int tf_pool_submit(tf_pool p, int solver, int prec, int n, int64_t nn
   r->t_submit = Clock::now();
   p->live[r->id] = r;
   ++p->submitted;
-  // What the resident solve or the ICC sweeps keep besides (a request that
-  // the matrix and its vectors leave room for is not refused over these).
-  if (r->bytes <= p->budget)
-    r->bytes = std::min(p->budget, r->bytes + (prec == TF_PREC_ICC ? tf_icc_bytes(n, nnz)
-                                                                    : tf_resident_bytes(n, nnz)));
+  // What the one-kernel solve or the ICC sweeps keep besides, as far as the
+  // budget has room for it: a request that the matrix and its vectors fit is
+  // not refused over these, but solved without them.
+  if (r->bytes <= p->budget) {
+    r->extra = std::min(p->budget - r->bytes, extra);
+    r->bytes += r->extra;
+  }
   if (r->bytes > p->budget) {      // can never be admitted
     r->status = TF_ERR_OOM;
     r->done = true;

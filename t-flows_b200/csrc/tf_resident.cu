@@ -494,31 +494,58 @@ constexpr size_t kResSmemMax = 225 * 1024 - 2048;   // beside the exchange's sta
 
 }  // namespace
 
-// Rows a CTA and the kernel's shape, when the matrix may fit the chip; otherwise
-// m->res.rows stays 0.  row0: its row pointers on the host.
-void tf_resident_plan(tf_matrix_s* m, const int* row0) {
-  const int n = m->ni, sms = m->ctx->sm_count;
-  m->res.rows = 0;
-  // (Buffer cells are rows that no CTA would own.)
-  if (n < 1 || m->nt != n) return;
+namespace {
+
+// Rows a CTA, the kernel's shape and the most entries of a CTA of a matrix that
+// may fit the chip; rows = 0: it does not.  row: row pointers, from any base.
+struct ResPlan {
+  int rows = 0, shape = 0, cap_ne = 0;
+};
+ResPlan res_plan(int n, const int* row, int sms) {
+  ResPlan p;
+  if (n < 1 || res_bits(n) > kResSmemMax) return p;
   // Rows a CTA: 256 (one a thread) while there are SMs for that many CTAs,
   // then as many as it takes (512 at the least: us an iteration at 27,000
   // rows 5.44 / 5.56 / 5.94 with 256 / 512 / 1024 rows a CTA).
   int rows = 256;
   if ((n + rows - 1) / rows > sms) rows = std::max(512, (n + sms - 1) / sms);
-  int shape = 0;
-  while (shape < kResShapeCount && kResShapes[shape].rpt * kResShapes[shape].threads < rows)
-    ++shape;
-  if (shape == kResShapeCount) return;
-  const int G = (n + rows - 1) / rows;
-  int cap_ne = 0;
-  for (int c = 0; c < G; ++c)
-    cap_ne = std::max(cap_ne, row0[std::min(n, (c + 1) * rows)] - row0[c * rows]);
-  if (cap_ne > 65535 || res_smem(cap_ne, rows, 0, rows) > kResSmemMax) return;
-  if (res_bits(n) > kResSmemMax) return;
-  m->res.rows = rows;
-  m->res.shape = shape;
-  m->res.cap_ne = (cap_ne + 7) & ~7;   // keeps what follows aligned
+  while (p.shape < kResShapeCount && kResShapes[p.shape].rpt * kResShapes[p.shape].threads < rows)
+    ++p.shape;
+  if (p.shape == kResShapeCount) return p;
+  for (int r0 = 0; r0 < n; r0 += rows)
+    p.cap_ne = std::max(p.cap_ne, row[std::min(n, r0 + rows)] - row[r0]);
+  if (p.cap_ne > 65535 || res_smem(p.cap_ne, rows, 0, rows) > kResSmemMax) return p;
+  p.cap_ne = (p.cap_ne + 7) & ~7;   // keeps what follows aligned
+  p.rows = rows;
+  return p;
+}
+
+// The layout's one allocation: words (sums, epoch, z), CTAs, halos, places.
+struct ResBytes {
+  size_t words, fixed, ctas, halo, slot;
+  ResBytes(int n, int64_t nnz, int G, int largest) {
+    auto up = [](size_t b) { return (b + 127) & ~size_t(127); };
+    words = (size_t)2 * G * kResWords * 8;
+    fixed = up(words + kResEpochBytes + (size_t)n * 16);
+    ctas = up(G * sizeof(ResCta));
+    halo = up((size_t)G * largest * 4 + 16);
+    slot = up((size_t)nnz * 2);
+  }
+  size_t total() const { return fixed + ctas + halo + slot; }
+};
+
+}  // namespace
+
+// At registration: whether the matrix may be solved by one kernel.  row0: its
+// row pointers on the host.  (TF_NO_RESIDENT keeps the graph of kernels, for
+// comparisons; buffer cells are rows that no CTA would own.)
+void tf_resident_plan(tf_matrix_s* m, const int* row0) {
+  m->res.rows = 0;
+  if (m->nt != m->ni || getenv("TF_NO_RESIDENT")) return;
+  const ResPlan p = res_plan(m->ni, row0, m->ctx->sm_count);
+  m->res.rows = p.rows;
+  m->res.shape = p.shape;
+  m->res.cap_ne = p.cap_ne;
 }
 
 namespace {
@@ -553,22 +580,20 @@ int res_build(tf_matrix_s* m) {
           &per_sm, f, kResShapes[shape].threads, smem));
       if (per_sm * sms < G) return TF_OK;   // all CTAs have to be resident at once
     }
-  // One allocation: words (sums, epoch, z), CTAs, halos, places.
-  auto up = [](size_t b) { return (b + 127) & ~size_t(127); };
-  const size_t words = (size_t)2 * G * kResWords * 8,
-               fixed = up(words + kResEpochBytes + (size_t)n * 16), ctab = up(G * sizeof(ResCta)),
-               hb = up((size_t)G * largest * 4 + 16), sb = up((size_t)m->nnz * 2);
+  const ResBytes bytes(n, m->nnz, G, largest);
+  if (m->extra_bytes + bytes.total() > m->extra_limit) return TF_OK;
   unsigned char* d = nullptr;
-  const int st = tf_dev_alloc_bytes(m->ctx, (void**)&d, fixed + ctab + hb + sb);
+  const int st = tf_dev_alloc_bytes(m->ctx, (void**)&d, bytes.total());
   if (st != TF_OK) return st;
+  m->extra_bytes += bytes.total();
   m->res.block = d;
   m->res.words = reinterpret_cast<unsigned long long*>(d);
-  m->res.epoch = reinterpret_cast<unsigned*>(d + words);
-  m->res.z = reinterpret_cast<unsigned long long*>(d + words + kResEpochBytes);
-  m->res.words_bytes = fixed;
-  m->res.cta = d + fixed;
-  m->res.halo = reinterpret_cast<int*>(d + fixed + ctab);
-  m->res.slot = reinterpret_cast<unsigned short*>(d + fixed + ctab + hb);
+  m->res.epoch = reinterpret_cast<unsigned*>(d + bytes.words);
+  m->res.z = reinterpret_cast<unsigned long long*>(d + bytes.words + kResEpochBytes);
+  m->res.words_bytes = bytes.fixed;
+  m->res.cta = d + bytes.fixed;
+  m->res.halo = reinterpret_cast<int*>(d + bytes.fixed + bytes.ctas);
+  m->res.slot = reinterpret_cast<unsigned short*>(d + bytes.fixed + bytes.ctas + bytes.halo);
   k_resident_build<<<G, 512, bits, s>>>(m->d_row, m->d_col, n, rows, largest,
                                         reinterpret_cast<ResCta*>(m->res.cta), m->res.halo,
                                         m->res.slot, nullptr);
@@ -597,10 +622,15 @@ int tf_resident_prepare(tf_matrix_s* m) {
   return st;
 }
 
-// Device bytes tf_resident_prepare may take, for budgeting.
-size_t tf_resident_bytes(int n, int64_t nnz) {
-  if (n < 1 || (size_t)nnz * 10 > (size_t)148 * kResSmemMax) return 0;
-  return (size_t)nnz * 2 + (size_t)n * 28 + ((size_t)1 << 16);
+// Device bytes the layout may take, for budgeting.  A CTA's halo has no more
+// rows than it has entries, or than fit its shared memory (a renumbered
+// matrix's entries a CTA are not known here).
+size_t tf_resident_bytes(int n, int64_t nnz, const int* row, bool renumbered, int sms) {
+  const ResPlan p = res_plan(n, row, sms);
+  if (p.rows == 0) return 0;
+  const int fits = (int)(kResSmemMax / 12);
+  return ResBytes(n, nnz, (n + p.rows - 1) / p.rows, renumbered ? fits : std::min(p.cap_ne, fits))
+      .total();
 }
 
 bool tf_resident(const tf_matrix_s* m) {

@@ -173,3 +173,48 @@ def test_pool_request_on_a_new_structure_is_not_passed_over_for_good(gpu_ctx):
             p.wait(rid)
     finally:
         p.close()
+
+
+@pytest.mark.parametrize("prec", ["jacobi", "icc"])
+def test_pool_budget_counts_what_makes_solves_faster(gpu_ctx, prec, monkeypatch):
+    """A budget with room for the matrix and its vectors but not for the
+    one-kernel solve's layout (or the ICC records): the request is solved
+    without, by the kernels a registration without them uses, and nothing
+    beyond the budget is held."""
+    s = systems.small_hex(24, seed=6, kind="pressure", ratio=1.02)
+    s = copy.copy(s)
+    s.prec = prec
+    full = _reference(gpu_ctx, s)
+    monkeypatch.setenv("TF_NO_RESIDENT", "1")
+    monkeypatch.setenv("TF_ICC_SWEEPS", "levels")
+    plain = _reference(gpu_ctx, s)
+    monkeypatch.delenv("TF_NO_RESIDENT")
+    monkeypatch.delenv("TF_ICC_SWEEPS")
+    assert not np.array_equal(plain[0], full[0])   # sums in another order
+
+    def served(budget):
+        p = pool.Pool(workers=1, mem_budget=budget)
+        try:
+            for _ in range(2):
+                r = p.wait(p.submit(s))
+            held = p.resident()
+            assert held["held"] == 1 and held["reused"] == 1
+            assert p.stats()["peak_bytes"] <= budget
+            return r, held["held_bytes"]
+        finally:
+            p.close()
+
+    r, most = served(1 << 30)
+    assert np.array_equal(r["x"], full[0])
+    least, _ = 0, None
+    lo, hi = 1 << 20, most
+    while hi - lo > 4096:       # the smallest budget that admits the request
+        mid = (lo + hi) // 2
+        try:
+            r, got = served(mid)
+            hi, least = mid, got
+            assert got <= mid
+        except native.TFError as e:
+            assert e.status == 2
+            lo = mid
+    assert least < most and np.array_equal(r["x"], plain[0])
