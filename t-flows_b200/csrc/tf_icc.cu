@@ -166,7 +166,6 @@ int pack(tf_matrix_s* m) {
     for (int k = 0; k < 2; ++k) {
       tf_icc_dir_s& g = m->icc_dir[k];
       cut_slices(*ptrs[k], slices[k], first[k]);
-      g.nlev = (int)ptrs[k]->size() - 1;
       g.nslices = (int)slices[k].size();
       const int nchunks = (g.nslices + kIccChunk - 1) / kIccChunk;
       st = dev_array(m, &g.slice, slices[k].size());
@@ -245,7 +244,6 @@ IccDir dir_args(const tf_icc_dir_s& g, const int* rows) {
   d.src = g.src;
   d.rec = g.rec;
   d.idx = g.idx;
-  d.nlev = g.nlev;
   d.nslices = g.nslices;
   d.far_any = g.far_any;
   return d;
@@ -367,7 +365,6 @@ int tf_icc_make_plan(tf_matrix_s* m, tf_icc_plan* p) {
   a.width = m->icc_width;
   a.stages = m->icc_stages;
   a.ring = m->icc_ring;
-  a.batch = m->icc_batch;
   if (m->icc_batch == 3) return plan_one<3, 3, 24>(m, p);
   if (m->icc_warps == 24) return plan_one<4, 4, 24>(m, p);
   return plan_one<12, 4, 16>(m, p);

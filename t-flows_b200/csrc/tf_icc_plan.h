@@ -43,7 +43,7 @@ struct IccDir {
   const int* src;        // packed entry -> entry of the matrix
   unsigned char* rec;    // the records
   const int* idx;        // row -> index of its right-hand side in rec (doubles)
-  int nlev, nslices;
+  int nslices;
   int far_any;           // results are read from global memory too
 };
 constexpr int kIccMetaBytes = kIccChunk * 32;
@@ -72,7 +72,7 @@ struct IccArgs {
   SolveState* st;
   const SolveParams* prm;
   IccDir f, b;           // forward and backward
-  int width, batch, stages, ring;
+  int width, stages, ring;
 };
 
 // One level's rows (one kernel per level).

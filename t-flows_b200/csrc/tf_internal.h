@@ -94,7 +94,7 @@ struct tf_icc_dir_s {
   int* src = nullptr;
   int* idx = nullptr;
   unsigned char* rec = nullptr;
-  int nlev = 0, nslices = 0, far_any = 0;
+  int nslices = 0, far_any = 0;
 };
 
 // The matrix's distribution over the CTAs of the resident solve
@@ -166,7 +166,7 @@ struct tf_matrix_s {
   long long icc_entries = 0;   // entries both sweeps visit
   int icc_long_levels = 0;     // levels with a row of more than kIccWidth of them
   double* d_icc_d = nullptr;     // Prec_Form's d
-  double* d_icc_dinv = nullptr;  // Prec_Form's d_inv
+  double* d_icc_dinv = nullptr;  // Prec_Form's d_inv (the kernels per level's)
   // The one-CTA sweeps' packed slices (tf_icc_prepare), made before the
   // first ICC solve of a matrix with narrow levels.
   tf_icc_dir_s icc_dir[2];       // forward, backward
