@@ -58,6 +58,15 @@ def golden_cases():
     return out
 
 
+@pytest.fixture(params=["one-kernel", "graph"])
+def solve_path(request, monkeypatch):
+    """Matrices that fit the chip registered for either form of the Jacobi /
+    none solve: one kernel, or the graph of kernels that larger ones take."""
+    if request.param == "graph":
+        monkeypatch.setenv("TF_NO_RESIDENT", "1")
+    return request.param
+
+
 @pytest.fixture(scope="session")
 def gpu_ctx():
     from tflows_b200 import native

@@ -5,7 +5,8 @@
   give up; the solve must end with TF_ERR_TIMEOUT (the CTAs still wait for
   the copies they started, with the default limit, before exiting), and
   the same context must then solve normally again.  Run on the row-pattern
-  streamer (hex) and on the CSR streamer (polyhedral).
+  streamer (hex) and on the CSR streamer (polyhedral), each in the graph of
+  kernels, and on the exchanges of the one-kernel solve of both.
 * Degenerate input the reference does not reject (Message_Mod/Error.f90 is
   never reached for it): NaN in b and a zero diagonal.  The numbers
   propagate; the drop-in must run the same iterations as the oracle (which
@@ -35,7 +36,7 @@ def gpu(ctx, m, s, val, b, miter, tol, norm, prec="jacobi"):
 
 
 @pytest.mark.parametrize("kind", ["hex-row-patterns", "poly-csr-tiles"])
-def test_wait_limit_runs_out_then_context_recovers(kind, monkeypatch):
+def test_wait_limit_runs_out_then_context_recovers(kind, solve_path, monkeypatch):
     if kind == "hex-row-patterns":
         s = systems.small_hex(64, seed=4, kind="pressure", ratio=1.02)
     else:
@@ -52,6 +53,7 @@ def test_wait_limit_runs_out_then_context_recovers(kind, monkeypatch):
             assert e.value.status == 4                     # TF_ERR_TIMEOUT
             ctx.set_wait_limit(0.0)                        # back to the default
             x, it, res = gpu(ctx, m, s, s.val, s.b, 5000, 1e-10, 1.0)
+            assert (m.resident_ctas > 0) == (solve_path == "one-kernel")
             ox, oit, ores = oracle(s, s.val, s.b, 5000, 1e-10, 1.0)
             assert abs(it - oit) <= max(1, 0.02 * oit) and res < 1e-10
             assert np.linalg.norm(x - ox) <= 1e-8 * np.linalg.norm(ox)
@@ -82,6 +84,48 @@ def test_icc_solve_that_times_out_leaves_the_next_solves_alone():
     finally:
         m.close()
         ctx.close()
+
+
+def test_icc_sweep_wait_runs_out_then_context_recovers(monkeypatch):
+    """One row of 5,000 lower entries is summed for some 2 ms while all other
+    warps of the sweep wait for it: under a limit of 0.1 ms they give up (the
+    products of such a matrix wait for nothing), under the default the solve is
+    the oracle's."""
+    monkeypatch.setenv("TF_ICC_SWEEPS", "one")
+    n, hub = 6000, 5000
+    rng = np.random.default_rng(8)
+    other = np.delete(np.arange(n), hub)
+    w = -rng.uniform(0.2, 1.0, n - 1)   # entries (hub, other) and (other, hub)
+    i = np.arange(n)
+    diag = np.full(n, 0.3)
+    diag[other] -= w
+    diag[hub] -= w.sum()
+    r, c, v = (np.concatenate(t) for t in ((i, np.full(n - 1, hub), other),
+                                           (i, other, np.full(n - 1, hub)), (diag, w, w)))
+    order = np.lexsort((c, c != r, r))
+    row = np.concatenate([[1], 1 + np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+    col, dia, val = (c[order] + 1).astype(np.int32), row[:-1].copy(), v[order]
+    b = rng.uniform(-1, 1, n)
+    ox, ov, ob = np.zeros(n), val.copy(), b.copy()
+    want = O.solve_native("cg", "icc", row, col, dia, ov, ox, ob, 20, 1e-10, norm=1.0)
+    with native.Context(0) as ctx:
+        m = native.Matrix(ctx, row, col, dia)
+        try:
+            assert m.tile_config == 3 and m.icc_kernels == 1
+            for _ in range(2):
+                ctx.set_wait_limit(1e-4)
+                with pytest.raises(native.TFError) as e:
+                    native.solve(ctx, m, "cg", "icc", val.copy(), np.zeros(n), b.copy(), 20,
+                                 1e-10, 1.0)
+                assert e.value.status == 4
+                ctx.set_wait_limit(0.0)
+                x = np.zeros(n)
+                it, res = native.solve(ctx, m, "cg", "icc", val.copy(), x, b.copy(), 20, 1e-10,
+                                       1.0)
+                assert it == want["niter"] and res < 1e-10
+                assert np.linalg.norm(x - ox) <= 1e-8 * np.linalg.norm(ox)
+        finally:
+            m.close()
 
 
 def test_icc_sweeps_longer_than_the_limit_run_to_their_end():
@@ -272,7 +316,7 @@ def same_propagation(g, o):
 
 
 @pytest.mark.parametrize("n", [6, 40])
-def test_nan_in_rhs_propagates_like_the_reference(gpu_ctx, n):
+def test_nan_in_rhs_propagates_like_the_reference(gpu_ctx, solve_path, n):
     s = systems.small_hex(n, seed=6, kind="pressure")
     b = s.b.copy()
     b[s.n // 3] = np.nan
@@ -287,7 +331,7 @@ def test_nan_in_rhs_propagates_like_the_reference(gpu_ctx, n):
 
 
 @pytest.mark.parametrize("prec", ["jacobi", "none"])
-def test_zero_diagonal_propagates_like_the_reference(gpu_ctx, prec):
+def test_zero_diagonal_propagates_like_the_reference(gpu_ctx, solve_path, prec):
     s = systems.small_hex(6, seed=7, kind="pressure")
     val = s.val.copy()
     val[s.csr.dia[11] - 1] = 0.0

@@ -19,7 +19,7 @@ def _single(ctx, m, s, prec, b, x0, miter, tol, norm):
 @pytest.mark.parametrize("prec", ["jacobi", "none"])
 @pytest.mark.parametrize("norm", [1.0, None])
 @pytest.mark.parametrize("nrhs", [1, 3, 4])
-def test_multi_rhs_equals_single_solves_bitwise(gpu_ctx, prec, norm, nrhs):
+def test_multi_rhs_equals_single_solves_bitwise(gpu_ctx, solve_path, prec, norm, nrhs):
     s = systems.small_hex(21, seed=4, kind="momentum", peclet=1.0, ratio=1.02)
     rng = np.random.default_rng(7)
     B = np.ascontiguousarray(rng.uniform(-1, 1, (nrhs, s.n)))
@@ -32,6 +32,7 @@ def test_multi_rhs_equals_single_solves_bitwise(gpu_ctx, prec, norm, nrhs):
         ref = [_single(gpu_ctx, m, s, prec, B[i], X0[i], 2000, 1e-10, norm) for i in range(nrhs)]
         val, X, Bm = s.val.copy(), X0.copy(), B.copy()
         its, res = native.solve_multi(gpu_ctx, m, "bicg", prec, val, X, Bm, 2000, 1e-10, norm)
+        assert (m.resident_ctas > 0) == (solve_path == "one-kernel")
     finally:
         m.close()
     for i in range(nrhs):
@@ -41,7 +42,7 @@ def test_multi_rhs_equals_single_solves_bitwise(gpu_ctx, prec, norm, nrhs):
         assert np.array_equal(val, v)
 
 
-def test_multi_rhs_early_exits_and_miter(gpu_ctx):
+def test_multi_rhs_early_exits_and_miter(gpu_ctx, solve_path):
     """A zero right-hand side stops at iteration 0 with fin_res 0 (Cg.f90:101-104)
     while the others run; miter caps each one."""
     s = systems.small_hex(15, seed=2, kind="pressure", ratio=1.03)
@@ -57,19 +58,23 @@ def test_multi_rhs_early_exits_and_miter(gpu_ctx):
     assert its == [7, 0, 7] and res[1] == 0.0 and np.all(X[1] == 0.0)
 
 
-def test_multi_rhs_on_csr_matrices_matches_oracle(gpu_ctx):
-    """Without row patterns (polyhedral mesh) the matrix is read by a
-    thread-per-row SpMV: same row sums, dot products in another order."""
-    g = grids.poly_lattice_grid(4000, 9)
+@pytest.mark.parametrize("cells", [4000, 20000])
+def test_multi_rhs_on_csr_matrices_matches_oracle(gpu_ctx, solve_path, cells):
+    """Without row patterns (polyhedral mesh) the graph reads the matrix by a
+    thread-per-row SpMV: same row sums, dot products in another order.  A
+    matrix with a renumbered copy is solved by the graph on the given
+    numbering."""
+    g = grids.poly_lattice_grid(cells, 9)
     s = systems.momentum_system(g, 9, tol=1e-10, miter=3000, peclet=5.0, cfl=0.1)
     rng = np.random.default_rng(1)
     B = np.ascontiguousarray(rng.uniform(-1, 1, (3, s.n)))
     X = np.zeros_like(B)
     m = native.Matrix(gpu_ctx, s.csr.row, s.csr.col, s.csr.dia)
     try:
-        assert m.row_patterns == 0
+        assert m.row_patterns == 0 and m.renumbered == (cells == 20000)
         its, res = native.solve_multi(gpu_ctx, m, "bicg", "jacobi", s.val.copy(), X, B.copy(),
                                       3000, 1e-10, 1.0)
+        assert (m.resident_ctas > 0) == (solve_path == "one-kernel" and cells == 4000)
     finally:
         m.close()
     for i in range(3):

@@ -84,7 +84,7 @@ def check_parity(g, o, tol, exact_iters=False):
 
 
 @pytest.mark.parametrize("case", golden_cases(), ids=lambda c: c["name"])
-def test_golden_fixture_parity(gpu_ctx, case):
+def test_golden_fixture_parity(gpu_ctx, solve_path, case):
     g = gpu_solve(gpu_ctx, case["row"], case["col"], case["dia"], case["val"], case["b"],
                   case["x0"], case["solver"], case["prec"], case["miter"], case["tol"],
                   case["norm"])
@@ -185,6 +185,7 @@ def test_variable_tiles_bitwise(gpu_ctx, mesh, n, cfg, monkeypatch):
     with the oracle (dot products are summed in another order per layout)."""
     torch = torch_dev()
     monkeypatch.setenv("TF_TILE_CFG", str(cfg))
+    monkeypatch.setenv("TF_NO_RESIDENT", "1")   # the whole solve on these tiles, too
     s = (systems.poly_system(n, seed=8, kind="pressure", tol=1e-10, miter=5000, norm=1.0)
          if mesh == "delaunay" else _lattice_poly(n, 8))
     rng = np.random.default_rng(9)
@@ -240,6 +241,7 @@ def test_row_patterns_do_not_change_the_solve(gpu_ctx, prec, norm, monkeypatch):
     every row sum, so a whole solve is bit-identical with the CSR columns on
     the same tiles (512-row tiles for both)."""
     monkeypatch.setenv("TF_TILE_CFG", "0")
+    monkeypatch.setenv("TF_NO_RESIDENT", "1")   # which reads no tiles
     s = systems.small_hex(23, seed=9, kind="pressure", ratio=1.04)
     args = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b, s.x0, "cg", prec, 3000, 1e-10, norm)
     g1 = gpu_solve(gpu_ctx, *args)
@@ -279,7 +281,7 @@ def test_renumbering_is_chosen_for_scattered_numberings(gpu_ctx, monkeypatch):
 
 
 @pytest.mark.parametrize("prec,norm", [("jacobi", 1.0), ("jacobi", None), ("none", 1.0)])
-def test_renumbered_solve_parity(gpu_ctx, prec, norm, monkeypatch):
+def test_renumbered_solve_parity(gpu_ctx, solve_path, prec, norm, monkeypatch):
     """Solves on the renumbered copy agree with the oracle (original order)
     and with the solve on the given numbering: same rows, same sums; only
     the dot products are summed in another order."""
@@ -299,7 +301,7 @@ def test_renumbered_solve_parity(gpu_ctx, prec, norm, monkeypatch):
 
 
 @pytest.mark.parametrize("miter", [1, 5])
-def test_renumbered_fin_res_is_nrms_of_returned_x(gpu_ctx, miter):
+def test_renumbered_fin_res_is_nrms_of_returned_x(gpu_ctx, solve_path, miter):
     s = _lattice_poly(20000, 7)
     x0 = np.random.default_rng(8).uniform(-0.5, 0.5, s.n)
     m = native.Matrix(gpu_ctx, s.csr.row, s.csr.col, s.csr.dia)
@@ -336,7 +338,7 @@ def test_buffer_cells(gpu_ctx, prec, norm):
     assert np.array_equal(x[ni:], x0[ni:])   # halo values untouched
 
 
-def test_long_rows_fall_back_to_global_path(gpu_ctx):
+def test_long_rows_fall_back_to_global_path(gpu_ctx, solve_path):
     """A row longer than any tile stage (a dense coupling row) still works."""
     n = 6000
     rows, cols = [], []
@@ -365,7 +367,7 @@ def test_long_rows_fall_back_to_global_path(gpu_ctx):
 @pytest.mark.parametrize("prec", ["jacobi", "none"])
 @pytest.mark.parametrize("norm", [None, 1.0])
 @pytest.mark.parametrize("m", [11, 12])   # odd and even cell counts
-def test_solve_variants_small(gpu_ctx, solver, prec, norm, m):
+def test_solve_variants_small(gpu_ctx, solve_path, solver, prec, norm, m):
     s = systems.small_hex(m, seed=6, kind="pressure", ratio=1.03)
     x0 = np.random.default_rng(4).uniform(-0.5, 0.5, s.n)
     args = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b, x0, solver, prec, 2000, 1e-10, norm)
@@ -376,7 +378,7 @@ def test_solve_variants_small(gpu_ctx, solver, prec, norm, m):
 @pytest.mark.parametrize("norm", [None, 1.0])
 @pytest.mark.parametrize("kind,m", [("hex", 11), ("hex", 64), ("poly", 3001)])
 @pytest.mark.parametrize("miter", [1, 2, 7])
-def test_fin_res_is_nrms_of_returned_x(gpu_ctx, prec, norm, kind, m, miter):
+def test_fin_res_is_nrms_of_returned_x(gpu_ctx, solve_path, prec, norm, kind, m, miter):
     """After a few iterations (no drift between the updated and the true
     residual yet) fin_res equals NRMS(b - A x) of the returned x to rounding:
     checks the device reductions and that x holds every update, including
@@ -396,7 +398,7 @@ def test_fin_res_is_nrms_of_returned_x(gpu_ctx, prec, norm, kind, m, miter):
     assert rel_l2(g[0], o[0]) <= 1e-12 and g[4] == pytest.approx(o[4], rel=1e-11)
 
 
-def test_bicg_equals_cg_on_gpu(gpu_ctx):
+def test_bicg_equals_cg_on_gpu(gpu_ctx, solve_path):
     s = systems.small_hex(16, seed=7, kind="momentum", peclet=1.0, ratio=1.02)
     a = (s.csr.row, s.csr.col, s.csr.dia, s.val, s.b, s.x0)
     g1 = gpu_solve(gpu_ctx, *a, "cg", "jacobi", 1000, 1e-10, 1.0)
@@ -437,7 +439,7 @@ def test_poly_parity(gpu_ctx):
     check_parity(gpu_solve(gpu_ctx, *args), oracle_solve(*args), 1e-10)
 
 
-def test_early_exits(gpu_ctx):
+def test_early_exits(gpu_ctx, solve_path):
     s = systems.small_hex(6, seed=2, kind="pressure")
     a = (s.csr.row, s.csr.col, s.csr.dia)
     # b == 0 -> niter 0, fin_res exactly 0.0, x untouched
@@ -513,7 +515,7 @@ def test_solve_device_pointers(gpu_ctx):
 
 @pytest.mark.parametrize("kind,prec,norm", [("hex", "jacobi", 1.0), ("hex", "none", None),
                                              ("hex", "icc", 1.0), ("poly", "jacobi", 1.0)])
-def test_solve_device_in_place_equals_host_solve(gpu_ctx, kind, prec, norm):
+def test_solve_device_in_place_equals_host_solve(gpu_ctx, solve_path, kind, prec, norm):
     """tf_solve_device works on the caller's arrays (16-byte aligned: in
     place; renumbered matrices gather from and scatter to them) and gives
     the bits of tf_solve; a second set of arrays rebuilds its graph, and
@@ -544,7 +546,7 @@ def test_solve_device_in_place_equals_host_solve(gpu_ctx, kind, prec, norm):
         m.close()
 
 
-def test_history_matches_oracle(gpu_ctx):
+def test_history_matches_oracle(gpu_ctx, solve_path):
     s = systems.small_hex(9, seed=5, kind="pressure")
     gpu_ctx.set_history(True)
     try:
@@ -746,7 +748,16 @@ def test_resident_solve_at_its_edges(gpu_ctx, case, prec, norm):
     n = len(a[4])
     x0 = np.random.default_rng(4).uniform(-0.5, 0.5, n)
     args = (*a, x0, "cg", prec, 9, 1e-300, norm)
-    g, o = gpu_solve(gpu_ctx, *args), oracle_solve(*args)
+    m = native.Matrix(gpu_ctx, *a[:3])
+    try:
+        v, x, b = a[3].copy(), x0.copy(), a[4].copy()
+        it, res = native.solve(gpu_ctx, m, "cg", prec, v, x, b, 9, 1e-300, norm)
+        rows = 256 if n <= 256 * 148 else max(512, -(-n // 148))
+        fits = case not in ("halo-too-large", "too-large-hex")
+        assert m.resident_ctas == (-(-n // rows) if fits else 0)
+    finally:
+        m.close()
+    g, o = (x, v, b, it, res), oracle_solve(*args)
     assert g[3] == o[3] and rel_l2(g[0], o[0]) <= 1e-12
     # The recursive residual after 9 steps: its rounding, about 9 eps |x0|-sized
     # terms a row, is 1e-13 of the first residual; on one row it is all rounding.

@@ -30,7 +30,7 @@ def _reference(ctx, s):
         m.close()
 
 
-def test_pool_matches_single_solves(gpu_ctx):
+def test_pool_matches_single_solves(gpu_ctx, solve_path):
     sysl = _systems()
     ref = [_reference(gpu_ctx, s) for s in sysl]
     p = pool.Pool(workers=4, mem_budget=1 << 30)
@@ -75,10 +75,11 @@ def test_pool_budget(gpu_ctx):
         p.close()
 
 
-def test_pool_reuses_resident_structures(gpu_ctx):
+def test_pool_reuses_resident_structures(gpu_ctx, solve_path):
     """Requests on the same Matrix_Type arrays run on the held registration
     (no re-registration) and give the single-solve results every time, also
-    with fresh right-hand sides."""
+    with fresh right-hand sides, whichever worker's stream its kernel or its
+    graph runs on."""
     s = systems.small_hex(20, seed=7, kind="pressure", ratio=1.03)
     rhs = [systems.uniform_rhs(s.n, 100 + k, zero_mean=True) for k in range(6)]
     refs = []
