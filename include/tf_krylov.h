@@ -165,8 +165,9 @@ int tf_solve_native(tf_ctx ctx, tf_matrix m, const char* solver,
  * arrays are) the solve runs on them in place: the first call with a new
  * set of arrays builds the solve's CUDA graph on them, later calls with the
  * same arrays reuse it (a Jacobi or unpreconditioned solve of a matrix that
- * fits the chip is one kernel and needs no graph).  val is then read in 16-byte units, so up to 8
- * bytes past its last entry are read (inside any cudaMalloc allocation).
+ * fits the chip is one kernel and needs no graph).  val is then read in
+ * 16-byte units, so up to 8 bytes past its last entry are read (inside any
+ * cudaMalloc allocation).
  * Arrays off a 16-byte boundary are copied into the matrix's own buffers
  * and back (same results). */
 int tf_solve_device(tf_ctx ctx, tf_matrix m, int solver, int prec,
@@ -182,8 +183,11 @@ int tf_solve_device(tf_ctx ctx, tf_matrix m, int solver, int prec,
  * niter[i], fin_res[i], x_i and b_i are those of tf_solve on (val, x_i,
  * b_i), bit for bit on row-pattern matrices (on other matrices to the
  * rounding of the dot products) -- while one SpMV per iteration reads the
- * matrix once for all of them.  val is scaled and returned once.  ICC is
- * not offered here (TF_ERR_ARG).  No reference counterpart. */
+ * matrix once for all of them; on a matrix that fits the chip (and has no
+ * renumbered copy) they are solved one after another by the one-kernel
+ * solve.  val is scaled and returned once.  After TF_ERR_TIMEOUT x may hold
+ * solved and unsolved right-hand sides.  ICC is not offered here
+ * (TF_ERR_ARG).  No reference counterpart. */
 int tf_solve_multi(tf_ctx ctx, tf_matrix m, int solver, int prec, int nrhs,
                    double* val, double* x, double* b, int miter, int* niter,
                    double tol, double* fin_res, const double* norm);

@@ -336,6 +336,8 @@ constexpr int kIccSmemBytes = 225 * 1024;
 //   hex 76^3      1,942  5,750   2481 / 1796   1.0 M           1,067  7,340  25489 / 17707
 //   hex 92^3      2,842  8,430   4089 / 3907   1.4 M           1,319  9,090  29612 / 23660
 //   hex 100^3     3,356  9,970   4664 / 5689   2.0 M           1,674 11,560  33927 / 34502
+// The lines lie below both kinds' crossing (hex 2,900 rows, polyhedral 11,300
+// entries); short rows of other numberings were measured up to 2,000 a level.
 constexpr long long kIccOneRows = 2000, kIccOneEntries = 11000;
 // ... and where more than an eighth of the levels hold a row with more entries
 // than are packed (kIccWidth): such a row is summed from global memory, about as
@@ -359,9 +361,9 @@ constexpr long long kIccOneLongEntries = 4000;
 // (progress >= first slice of its level: slices of its own level or later
 // ones cannot have been counted before).
 //
-// Measured (57x43x53 hex, 302 levels of 27 slices): 331 us for both sweeps, 166
-// instructions a slice, the SM's issue slots and its shared-memory pipe each
-// about 60 % busy; a level alone takes about 0.5 us (poll, gather, sum,
+// Measured (57x43x53 hex, 302 levels of 27 slices): 329 us for both sweeps, 160
+// instructions a slice, the SM's issue slots 52 % and its shared-memory pipe
+// 64 % busy; a level alone takes about 0.5 us (poll, gather, sum,
 // store, report).  Copying a chunk's arrays one by one, with divisions in the
 // producer's loop, made it 740 us: a bulk copy costs its issuing lane some
 // 150 cycles whatever its size.
