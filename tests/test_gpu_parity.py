@@ -317,7 +317,8 @@ def test_renumbered_fin_res_is_nrms_of_returned_x(gpu_ctx, solve_path, miter):
                                 rel=1e-9)
 
 
-@pytest.mark.parametrize("prec,norm", [("jacobi", 1.0), ("jacobi", None), ("none", 1.0)])
+@pytest.mark.parametrize("prec,norm", [("jacobi", 1.0), ("jacobi", None), ("none", 1.0),
+                                       ("icc", 1.0)])
 def test_buffer_cells(gpu_ctx, prec, norm):
     """n_own < n_cells, as on an MPI sub-domain (Cg.f90:54, ni = n_cells -
     n_buff_cells): rows beyond ni are not solved, their x values enter the
