@@ -669,7 +669,7 @@ int run_solve_core(tf_matrix_s* m, int prec, int miter, double tol,
     TF_CUDA_TRY(cudaMemcpyAsync(a->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));
   if (a != m) st = tf_renumber_in(m);
   if (st == TF_OK)
-    st = resident ? tf_resident_run(a, prec, hp, a->d_x, a->d_b, a->d_state, nullptr, 1)
+    st = resident ? tf_resident_run(a, prec, hp, a->d_x, a->d_b, a->d_state, 0, 1)
                   : tf_fp64_run(a, prec);
   if (st == TF_OK && a != m) st = tf_renumber_out(m);
   if (st != TF_OK) return st;
@@ -859,8 +859,7 @@ int run_multi_core(tf_matrix_s* m, int prec, int nrhs, int miter, double tol,
     for (int i = 0; i < nrhs && st == TF_OK; ++i)
       st = tf_resident_run(m, prec, hp, x ? x + (size_t)i * m->nt : rhs_x(m, i),
                            b ? b + (size_t)i * m->nt : rhs_b(m, i),
-                           const_cast<tf::SolveState*>(rhs_state(m, i)),
-                           i > 0 ? rhs_state(m, i - 1) : nullptr, i == nrhs - 1);
+                           const_cast<tf::SolveState*>(rhs_state(m, i)), i, i == nrhs - 1);
   } else {
     TF_CUDA_TRY(
         cudaMemcpyAsync(m->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));

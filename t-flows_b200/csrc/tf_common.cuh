@@ -343,9 +343,9 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, unsigned parit
 }
 // A deadline whose looks mostly read the SM clock only: the global timer is read
 // at the first look after the limit starts to count and then only when
-// kLookCycles have passed since, so a limit is kept to within that.  Once passed
-// it stays so until renewed: a wait that gave up early may leave it to the next
-// look to end the kernel.
+// kLookCycles have passed since, so a limit is kept to within that: a look that
+// answers true is not repeated for a while, and what it ends has to remember it
+// (give_up(): the next look answers true again).
 struct Deadline {
   unsigned long long limit, ns;   // globaltimer
   long long look;                 // SM clock at which to read it again
@@ -360,11 +360,10 @@ struct Deadline {
   __device__ __forceinline__ bool passed() {
     const long long c = clock64();
     if (c < look) return false;
-    if (globaltimer_ns() > ns) return true;   // and again at the next look
     look = c + kLookCycles;
-    return false;
+    return globaltimer_ns() > ns;
   }
-  // Passed, from now on (globaltimer is past 0).
+  // Passed at the next look (globaltimer is past 0).
   __device__ __forceinline__ void give_up() {
     ns = 0;
     look = 0;

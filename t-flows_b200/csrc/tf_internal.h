@@ -242,7 +242,7 @@ void tf_resident_plan(tf_matrix_s* m, const int* row0);   // at registration
 int tf_resident_prepare(tf_matrix_s* m);   // before a solve without ICC
 size_t tf_resident_bytes(int n, int64_t nnz, const int* row, bool renumbered, int sms);
 int tf_resident_run(tf_matrix_s* m, int prec, const tf::SolveParams* p, double* x, double* b,
-                    tf::SolveState* st, const tf::SolveState* before, int write_val);
+                    tf::SolveState* st, int queued, int write_val);
 int tf_resident_reset(tf_matrix_s* m);
 // Whether Jacobi / none solves of m, once prepared, run as one resident kernel.
 bool tf_resident(const tf_matrix_s* m);

