@@ -130,8 +130,8 @@ int tf_matrix_row_patterns(tf_matrix m);
  * No reference counterpart: a property of this library's device layout. */
 int tf_matrix_renumbered(tf_matrix m);
 /* CTAs of the one-kernel Jacobi / none solve of a matrix that fits the chip
- * (of its renumbered copy when it has one); 0 before the first such solve,
- * which lays it out, and for matrices that do not fit or have buffer cells.
+ * (of its renumbered copy when it has one); 0 for matrices that do not fit,
+ * that have buffer cells, or whose layout found no memory.
  * No reference counterpart. */
 int tf_matrix_resident(tf_matrix m);
 

@@ -427,6 +427,7 @@ int matrix_create_impl(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const
   m->max_row_len = max_len;
   m->diag_first = diag_first;
   m->async_alloc = ctx->async_alloc;
+  m->extra_limit = ctx->extra_limit;
   m->dev_bytes = tf_matrix_bytes(n_cells, nnz);
 
   std::vector<int> row0((size_t)n_cells + 1 + 8, 0), col0((size_t)nnz + 8, 0),
@@ -537,7 +538,8 @@ int matrix_create_impl(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const
   if (st == TF_OK && n_cells > 0 && diag_first && want_icc)
     st = tf_icc_build(m, row0.data(), col0.data());
   if (st == TF_OK && allow_renumber) st = attach_renumbered(m, row0, col0, dia0);
-  if (st == TF_OK && n_cells > 0 && !m->ren) tf_resident_plan(m, row0.data());
+  if (st == TF_OK && n_cells > 0 && !m->ren && want_icc != tf_icc_only)
+    st = tf_resident_prepare(m, row0.data());
   if (st != TF_OK) {
     tf_matrix_free(m);
     return st;
@@ -662,11 +664,10 @@ int run_solve_core(tf_matrix_s* m, int prec, int miter, double tol,
     hp->hist_cap = miter + 1;
   }
   if (prec == tf::kPrecIcc && !m->icc_ready) return TF_ERR_LAYOUT;  // needs diagonal first
-  int st = prec != tf::kPrecIcc ? tf_resident_prepare(a) : TF_OK;
-  if (st != TF_OK) return st;
   const bool resident = prec != tf::kPrecIcc && tf_resident(a);
   if (!resident)
     TF_CUDA_TRY(cudaMemcpyAsync(a->d_params, hp, sizeof(*hp), cudaMemcpyHostToDevice, c->stream));
+  int st = TF_OK;
   if (a != m) st = tf_renumber_in(m);
   if (st == TF_OK)
     st = resident ? tf_resident_run(a, prec, hp, a->d_x, a->d_b, a->d_state, 0, 1)
@@ -916,8 +917,7 @@ extern "C" int tf_solve_multi(tf_ctx ctx, tf_matrix m, int solver, int prec, int
   if (!val || !x || !b) return TF_ERR_ARG;
   std::lock_guard<std::mutex> lk(m->mu);
   TF_CUDA_TRY(cudaSetDevice(ctx->device));
-  st = tf_resident_prepare(m);
-  if (st == TF_OK) st = tf_slices_ensure(m, nrhs);
+  st = tf_slices_ensure(m, nrhs);
   if (st != TF_OK) return st;
   cudaStream_t s = ctx->stream;
   const size_t vb = (size_t)m->nnz * sizeof(double), nb = (size_t)m->nt * sizeof(double);
@@ -958,8 +958,7 @@ extern "C" int tf_solve_multi_device(tf_ctx ctx, tf_matrix m, int solver, int pr
   if (!d_val || !d_x || !d_b) return TF_ERR_ARG;
   std::lock_guard<std::mutex> lk(m->mu);
   TF_CUDA_TRY(cudaSetDevice(ctx->device));
-  st = tf_resident_prepare(m);
-  if (st == TF_OK) st = tf_slices_ensure(m, nrhs, tf_resident(m));
+  st = tf_slices_ensure(m, nrhs, tf_resident(m));
   if (st != TF_OK) return st;
   cudaStream_t s = ctx->stream;
   const size_t vb = (size_t)m->nnz * sizeof(double), nb = (size_t)m->nt * sizeof(double);

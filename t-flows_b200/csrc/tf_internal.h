@@ -68,6 +68,7 @@ struct tf_ctx_s {
   // for matrices registered on this context: set by the request pool so a
   // worker never synchronises the device when it registers or releases.
   int async_alloc = 0;
+  size_t extra_limit = SIZE_MAX;        // of the matrices registered next (tf_matrix_s)
   tf::SolveState* h_state = nullptr;    // pinned, lent to async matrices
   tf::SolveParams* h_params = nullptr;
 };
@@ -98,10 +99,9 @@ struct tf_icc_dir_s {
 };
 
 // The matrix's distribution over the CTAs of the resident solve
-// (tf_resident.cu), made before the first Jacobi / none solve; rows = 0: it
-// does not fit the chip.
+// (tf_resident.cu), made at registration; ctas = 0: it does not fit the chip
+// (or its memory does not fit the device).
 struct tf_resident_s {
-  int rows = 0;               // rows a CTA
   int ctas = 0, shape = 0, threads = 0;
   size_t smem = 0;
   int cap_ne = 0, cap_p = 0, cap_halo = 0;
@@ -238,13 +238,12 @@ int tf_fp64_residual(tf_matrix_s* m, const double* val, const double* b,
                      const double* x, double* r);
 int tf_fp64_nrms(tf_matrix_s* m, const double* val, const double* r,
                  const double* x, int has_norm, double norm, double* out);
-void tf_resident_plan(tf_matrix_s* m, const int* row0);   // at registration
-int tf_resident_prepare(tf_matrix_s* m);   // before a solve without ICC
+int tf_resident_prepare(tf_matrix_s* m, const int* row0);   // at registration
 size_t tf_resident_bytes(int n, int64_t nnz, const int* row, bool renumbered, int sms);
 int tf_resident_run(tf_matrix_s* m, int prec, const tf::SolveParams* p, double* x, double* b,
                     tf::SolveState* st, int queued, int write_val);
 int tf_resident_reset(tf_matrix_s* m);
-// Whether Jacobi / none solves of m, once prepared, run as one resident kernel.
+// Whether Jacobi / none solves of m run as one resident kernel.
 bool tf_resident(const tf_matrix_s* m);
 int tf_icc_build(tf_matrix_s* m, const int* h_row0, const int* h_col0);
 int tf_icc_prepare(tf_matrix_s* m);   // before a solve with ICC
@@ -253,7 +252,9 @@ void tf_icc_free(tf_matrix_s* m);
 size_t tf_icc_bytes(int n, int64_t nnz);   // what the sweeps' records may take, for budgeting
 tf::IccResid tf_icc_resid(const tf_matrix_s* m);
 // Registration behind tf_matrix_register; want_icc = 0 skips the ICC level
-// schedule.  Device bytes the matrix will hold, for budgeting.
+// schedule, tf_icc_only the layout of solves without ICC.  Device bytes the
+// matrix will hold, for budgeting.
+constexpr int tf_icc_only = 2;
 int tf_matrix_create(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const int* row,
                      const int* col, const int* dia, int want_icc, tf_matrix_s** out);
 void tf_matrix_free(tf_matrix_s* m);

@@ -179,12 +179,11 @@ struct tf_pool_s {
     tf_matrix_s* m = *pm;
     int st = TF_OK;
     if (!m) {
-      st = tf_matrix_create(ctx, r.n, r.n, r.nnz, r.row, r.col, r.dia, r.prec == tf::kPrecIcc,
-                            &m);
+      ctx->extra_limit = r.extra;
+      st = tf_matrix_create(ctx, r.n, r.n, r.nnz, r.row, r.col, r.dia,
+                            r.prec == tf::kPrecIcc ? tf_icc_only : 0, &m);
       if (st != TF_OK) return st;
       *pm = m;
-      m->extra_limit = r.extra;
-      if (m->ren) m->ren->extra_limit = r.extra;
     }
     cudaStream_t s = ctx->stream;
     const size_t vb = (size_t)r.nnz * 8, nb = (size_t)r.n * 8;

@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(T, 1) k_resident(ResArgs a) {
     for (int h = t + kResAhead * T; h < nh; h += T) {
       double z = 0.0;
       bool gone = false;
-      for (int spin = 0; !gone && !take(h, z, tag); ++spin)
+      for (int spin = 0; !take(h, z, tag) && !gone; ++spin)
         if ((spin & 63) == 63) gone = deadline.passed();
       if (gone) deadline.give_up();
       sp[nr + h] = direction(z, sp[nr + h]);
@@ -529,25 +529,13 @@ struct ResBytes {
 
 }  // namespace
 
-// At registration: whether the matrix may be solved by one kernel.  row0: its
-// row pointers on the host.  (TF_NO_RESIDENT keeps the graph of kernels, for
-// comparisons; buffer cells are rows that no CTA would own.)
-void tf_resident_plan(tf_matrix_s* m, const int* row0) {
-  m->res.rows = 0;
-  if (m->nt != m->ni || getenv("TF_NO_RESIDENT")) return;
-  const ResPlan p = res_plan(m->ni, row0, m->ctx->sm_count);
-  m->res.rows = p.rows;
-  m->res.shape = p.shape;
-  m->res.cap_ne = p.cap_ne;
-}
-
 namespace {
 
 // The CTAs' halos and the entries' places in p, made on the device from the
 // matrix's row and column arrays; m->res.ctas stays 0 when they do not fit.
-int res_build(tf_matrix_s* m) {
-  const int n = m->ni, sms = m->ctx->sm_count, rows = m->res.rows, shape = m->res.shape;
-  const int G = (n + rows - 1) / rows, cap_ne = m->res.cap_ne;
+int res_build(tf_matrix_s* m, const ResPlan& p) {
+  const int n = m->ni, sms = m->ctx->sm_count, rows = p.rows, shape = p.shape;
+  const int G = (n + rows - 1) / rows, cap_ne = p.cap_ne;
   const size_t bits = res_bits(n);
   cudaStream_t s = m->ctx->stream;
   TF_CUDA_TRY(cudaFuncSetAttribute(k_resident_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -591,8 +579,10 @@ int res_build(tf_matrix_s* m) {
                                         reinterpret_cast<ResCta*>(m->res.cta), m->res.halo,
                                         m->res.slot, nullptr);
   TF_CUDA_TRY(cudaGetLastError());
+  m->res.shape = shape;
   m->res.threads = kResShapes[shape].threads;
   m->res.smem = smem;
+  m->res.cap_ne = cap_ne;
   m->res.cap_p = cap_p;
   m->res.cap_halo = cap_halo;
   m->res.ctas = G;
@@ -601,13 +591,16 @@ int res_build(tf_matrix_s* m) {
 
 }  // namespace
 
-// Before a Jacobi / none solve: the first one of a matrix lays it out (a matrix
-// registered for other uses carries nothing of it).  Without room for that the
-// graph of kernels, which has its memory, solves the matrix.
-int tf_resident_prepare(tf_matrix_s* m) {
-  if (m->res.rows == 0 || m->res.ctas > 0) return TF_OK;
-  int st = res_build(m);
-  if (m->res.ctas == 0) m->res.rows = 0;   // does not fit
+// At registration, where the matrix may be solved by one kernel (row0: its row
+// pointers on the host).  Without room for the layout the graph of kernels, which
+// has its memory, solves the matrix.  (Made by the first solve instead, solves of
+// 27,000 rows took 1 to 2 % longer on the later allocation.  TF_NO_RESIDENT keeps
+// the graph, for comparisons; buffer cells are rows that no CTA would own.)
+int tf_resident_prepare(tf_matrix_s* m, const int* row0) {
+  if (m->nt != m->ni || getenv("TF_NO_RESIDENT")) return TF_OK;
+  const ResPlan p = res_plan(m->ni, row0, m->ctx->sm_count);
+  if (p.rows == 0) return TF_OK;
+  int st = res_build(m, p);
   if (st == TF_ERR_OOM) {
     cudaGetLastError();   // not to be found by the next launch
     st = TF_OK;

@@ -298,8 +298,8 @@ class Matrix:
 
     @property
     def resident_ctas(self):
-        """CTAs of the one-kernel Jacobi / none solve (0: not laid out yet, or
-        the solve is a graph of kernels)."""
+        """CTAs of the one-kernel Jacobi / none solve (0: the solve is a graph
+        of kernels)."""
         return load().tf_matrix_resident(self.h)
 
     @property

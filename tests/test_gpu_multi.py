@@ -74,7 +74,7 @@ def test_multi_rhs_on_csr_matrices_matches_oracle(gpu_ctx, solve_path, cells):
         assert m.row_patterns == 0 and m.renumbered == (cells == 20000)
         its, res = native.solve_multi(gpu_ctx, m, "bicg", "jacobi", s.val.copy(), X, B.copy(),
                                       3000, 1e-10, 1.0)
-        assert (m.resident_ctas > 0) == (solve_path == "one-kernel" and cells == 4000)
+        assert (m.resident_ctas > 0) == (solve_path == "one-kernel")   # (of the copy)
     finally:
         m.close()
     for i in range(3):

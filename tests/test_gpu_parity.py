@@ -765,27 +765,3 @@ def test_resident_solve_at_its_edges(gpu_ctx, case, prec, norm):
     assert g[4] == pytest.approx(o[4], rel=1e-9, abs=1e-12 * n)
     assert np.allclose(g[1], o[1], rtol=4e-16, atol=0)
     assert np.allclose(g[2], o[2], rtol=4e-16, atol=0)
-
-
-def test_resident_layout_is_made_by_the_first_solve_that_uses_it(gpu_ctx):
-    """A matrix registered for products, assembly or ICC carries nothing of the
-    one-kernel solve."""
-    torch = torch_dev()
-    s = systems.small_hex(12, seed=3, kind="pressure")
-    d = _dev_arrays(torch, s.val, s.b, np.zeros(s.n))
-    torch.cuda.synchronize()
-    m = native.Matrix(gpu_ctx, s.csr.row, s.csr.col, s.csr.dia)
-    try:
-        def solve(prec):
-            v, x, b = s.val.copy(), s.x0.copy(), s.b.copy()
-            return native.solve(gpu_ctx, m, "cg", prec, v, x, b, 500, 1e-9, 1.0)
-
-        native.spmv(gpu_ctx, m, *(t.data_ptr() for t in d))
-        solve("icc")
-        gpu_ctx.sync()
-        assert m.resident_ctas == 0
-        first = solve("jacobi")
-        assert m.resident_ctas == (s.n + 255) // 256
-        assert solve("jacobi") == first
-    finally:
-        m.close()
