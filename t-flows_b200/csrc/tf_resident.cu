@@ -490,7 +490,8 @@ constexpr size_t kResSmemMax = 225 * 1024 - 2048;   // beside the exchange's sta
 namespace {
 
 // Rows a CTA, the kernel's shape and the most entries of a CTA of a matrix that
-// may fit the chip; rows = 0: it does not.  row: row pointers, from any base.
+// may fit the chip; rows = 0: it does not.  row: row pointers, from any base
+// (null: entries are not looked at).
 struct ResPlan {
   int rows = 0, shape = 0, cap_ne = 0;
 };
@@ -505,7 +506,7 @@ ResPlan res_plan(int n, const int* row, int sms) {
   while (p.shape < kResShapeCount && kResShapes[p.shape].rpt * kResShapes[p.shape].threads < rows)
     ++p.shape;
   if (p.shape == kResShapeCount) return p;
-  for (int r0 = 0; r0 < n; r0 += rows)
+  for (int r0 = 0; row && r0 < n; r0 += rows)
     p.cap_ne = std::max(p.cap_ne, row[std::min(n, r0 + rows)] - row[r0]);
   if (p.cap_ne > 65535 || res_smem(p.cap_ne, rows, 0, rows) > kResSmemMax) return p;
   p.cap_ne = (p.cap_ne + 7) & ~7;   // keeps what follows aligned
@@ -612,7 +613,7 @@ int tf_resident_prepare(tf_matrix_s* m, const int* row0) {
 // rows than it has entries, or than fit its shared memory (a renumbered
 // matrix's entries a CTA are not known here).
 size_t tf_resident_bytes(int n, int64_t nnz, const int* row, bool renumbered, int sms) {
-  const ResPlan p = res_plan(n, row, sms);
+  const ResPlan p = res_plan(n, renumbered ? nullptr : row, sms);
   if (p.rows == 0) return 0;
   const int fits = (int)(kResSmemMax / 12);
   return ResBytes(n, nnz, (n + p.rows - 1) / p.rows, renumbered ? fits : std::min(p.cap_ne, fits))
