@@ -537,7 +537,8 @@ int matrix_create_impl(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const
   }
   if (st == TF_OK && n_cells > 0 && diag_first && want_icc)
     st = tf_icc_build(m, row0.data(), col0.data());
-  if (st == TF_OK && allow_renumber) st = attach_renumbered(m, row0, col0, dia0);
+  if (st == TF_OK && allow_renumber && want_icc != tf_icc_only)
+    st = attach_renumbered(m, row0, col0, dia0);
   if (st == TF_OK && n_cells > 0 && !m->ren && want_icc != tf_icc_only)
     st = tf_resident_prepare(m, row0.data());
   if (st != TF_OK) {

@@ -252,8 +252,8 @@ void tf_icc_free(tf_matrix_s* m);
 size_t tf_icc_bytes(int n, int64_t nnz);   // what the sweeps' records may take, for budgeting
 tf::IccResid tf_icc_resid(const tf_matrix_s* m);
 // Registration behind tf_matrix_register; want_icc = 0 skips the ICC level
-// schedule, tf_icc_only the layout of solves without ICC.  Device bytes the
-// matrix will hold, for budgeting.
+// schedule, tf_icc_only what solves without ICC run on (the renumbered copy, the
+// one-kernel layout).  Device bytes the matrix will hold, for budgeting.
 constexpr int tf_icc_only = 2;
 int tf_matrix_create(tf_ctx_s* ctx, int n_cells, int n_own, int64_t nnz, const int* row,
                      const int* col, const int* dia, int want_icc, tf_matrix_s** out);

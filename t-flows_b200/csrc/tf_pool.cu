@@ -337,8 +337,7 @@ extern "C" int tf_pool_submit(tf_pool p, int solver, int prec, int n, int64_t nn
       prec == TF_PREC_ICC
           ? tf_icc_bytes(n, nnz)
           : tf_resident_bytes(n, nnz, row, made > plain, p->ctxs[0]->sm_count);
-  r->bytes = made +
-             (prec == TF_PREC_ICC ? (size_t)n * 40 + 4096 : 0);
+  r->bytes = prec == TF_PREC_ICC ? plain + (size_t)n * 40 + 4096 : made;
   r->key = structure_key(n, nnz, row, col, dia, prec == TF_PREC_ICC);
   std::lock_guard<std::mutex> lk(p->mu);
   if (p->stop) return TF_ERR_CANCELLED;

@@ -7,7 +7,7 @@ import threading
 import numpy as np
 import pytest
 
-from tflows_b200 import native, pool, systems
+from tflows_b200 import grids, native, pool, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -219,3 +219,26 @@ def test_pool_budget_counts_what_makes_solves_faster(gpu_ctx, prec, monkeypatch)
             assert e.status == 2
             lo = mid
     assert least < most and np.array_equal(r["x"], plain[0])
+
+
+def test_pool_icc_request_on_a_scattered_numbering(gpu_ctx):
+    """The registration of an ICC request leaves out the renumbered copy, which
+    ICC does not use; what it holds is what the budget counts."""
+    s = copy.copy(systems.pressure_system(grids.poly_lattice_grid(12000, 4), 4, tol=1e-9,
+                                          miter=300))
+    s.prec = "icc"
+    want = _reference(gpu_ctx, s)
+    p = pool.Pool(workers=2, mem_budget=1 << 30)
+    try:
+        r = p.wait(p.submit(s))
+        assert r["niter"] == want[1] and np.array_equal(r["x"], want[0])
+        held = p.resident()
+        s.prec = "jacobi"
+        p.wait(p.submit(s))
+        both = p.resident()
+    finally:
+        p.close()
+    n, nnz = s.n, s.nnz
+    matrix = 12 * nnz + 8 * n + 6 * 8 * n   # values, columns, rows, diagonals, vectors
+    assert matrix < held["held_bytes"] < 2 * matrix + 32 * nnz + 300 * n
+    assert both["held_bytes"] - held["held_bytes"] > 2 * matrix   # the copy, too
