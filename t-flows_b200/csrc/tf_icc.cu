@@ -37,40 +37,42 @@ int tf_icc_build(tf_matrix_s* m, const int* row0, const int* col0) {
   const int ni = m->ni;
   std::vector<int> levf(ni, 0), levb(ni, 0);
   int nf = 0, nb = 0;
-  // Entries the sweeps visit, and levels with a row longer than is packed.
-  std::vector<char> longf(ni, 0), longb(ni, 0);
-  m->icc_entries = 0;
-  auto count = [&](std::vector<char>& lev, int l, int len) {
-    m->icc_entries += len;
-    if (len > kIccWidth) lev[l] = 1;
-  };
+  // Entries the sweeps visit (with buffer cells'), and the levels of rows longer
+  // than is packed.
+  long long entries = 0;
+  std::vector<int> longf, longb;
   for (int i = 0; i < ni; ++i) {
-    int l = 0, len = 0;
-    for (int j = row0[i] + 1; j < row0[i + 1]; ++j) {
+    int l = 0, j = row0[i] + 1;
+    for (; j < row0[i + 1]; ++j) {
       const int k = col0[j];
       if (k > i) break;
       l = std::max(l, levf[k] + 1);
-      ++len;
     }
     levf[i] = l;
     nf = std::max(nf, l + 1);
-    count(longf, l, len);
+    const int len = j - row0[i] - 1;
+    entries += len;
+    if (len > kIccWidth) longf.push_back(l);
   }
   for (int i = ni - 1; i >= 0; --i) {
-    int l = 0, len = 0;
-    for (int j = row0[i + 1] - 1; j >= row0[i] + 1; --j) {
+    int l = 0, j = row0[i + 1] - 1;
+    for (; j >= row0[i] + 1; --j) {
       const int k = col0[j];
       if (k < i) break;
-      if (k >= ni) continue;
-      l = std::max(l, levb[k] + 1);
-      ++len;
+      if (k < ni) l = std::max(l, levb[k] + 1);
     }
     levb[i] = l;
     nb = std::max(nb, l + 1);
-    count(longb, l, len);
+    const int len = row0[i + 1] - 1 - j;
+    entries += len;
+    if (len > kIccWidth) longb.push_back(l);
   }
-  m->icc_long_levels = (int)(std::count(longf.begin(), longf.end(), 1) +
-                             std::count(longb.begin(), longb.end(), 1));
+  m->icc_entries = entries;
+  m->icc_long_levels = 0;
+  for (auto* lev : {&longf, &longb}) {
+    std::sort(lev->begin(), lev->end());
+    m->icc_long_levels += (int)(std::unique(lev->begin(), lev->end()) - lev->begin());
+  }
   std::vector<int> rf, rb;
   bucket(levf, nf, m->h_levf_ptr, rf);
   bucket(levb, nb, m->h_levb_ptr, rb);
